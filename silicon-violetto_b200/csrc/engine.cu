@@ -1523,10 +1523,10 @@ double Engine::spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t*
     const size_t pb = size_t(streams) * (k + 1) * vocab * 2, qb = size_t(streams) * k * vocab * 2;
     if (spec_p.bytes < pb) spec_p.alloc(pb, false);
     if (spec_q.bytes < qb) spec_q.alloc(qb, false);
-    // small: drafts | seeds | pos0 | accepted | token | rollback | row statistics
+    // small: drafts | seeds | pos0 | accepted | token | rollback | the rows' scratch
     const size_t o_seeds = (size_t(streams) * k * 4 + 255) / 256 * 256, o_pos = o_seeds + (size_t(streams) * 8 + 255) / 256 * 256;
     const size_t o_out = o_pos + (size_t(streams) * 4 + 255) / 256 * 256, o_stats = o_out + (size_t(streams) * 12 + 255) / 256 * 256;
-    const size_t small = o_stats + size_t(streams) * (2 * k + 1) * 16;
+    const size_t small = o_stats + size_t(streams) * (2 * k + 1) * sizeof(SpecRowWork);
     if (spec_small.bytes < small) spec_small.alloc(small, false);
     uint8_t* sm = spec_small.as<uint8_t>();
     VLT_CUDA(cudaMemcpyAsync(spec_p.dev, p, pb, cudaMemcpyHostToDevice, stream));
@@ -1541,9 +1541,9 @@ double Engine::spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t*
     uint32_t* o = reinterpret_cast<uint32_t*>(sm + o_out);
     for (uint32_t r = 0; r < std::max(reps, 1u); r++) {
         VLT_CUDA(cudaEventRecord(e0, stream));
-        launch_spec_accept(spec_p.as<uint16_t>(), spec_q.as<uint16_t>(), reinterpret_cast<const uint32_t*>(sm), streams, k, vocab, temperature,
-                           reinterpret_cast<const uint64_t*>(sm + o_seeds), reinterpret_cast<const uint32_t*>(sm + o_pos), sm + o_stats, o, o + streams,
-                           o + 2 * streams, stream);
+        VLT_CUDA(launch_spec_accept(spec_p.as<uint16_t>(), spec_q.as<uint16_t>(), reinterpret_cast<const uint32_t*>(sm), streams, k, vocab, temperature,
+                                    reinterpret_cast<const uint64_t*>(sm + o_seeds), reinterpret_cast<const uint32_t*>(sm + o_pos), reinterpret_cast<SpecRowWork*>(sm + o_stats), o, o + streams,
+                                    o + 2 * streams, stream));
         VLT_CUDA(cudaEventRecord(e1, stream));
         VLT_CUDA(cudaEventSynchronize(e1));
         float ms = 0;

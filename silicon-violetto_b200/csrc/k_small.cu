@@ -464,19 +464,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float* __r
                 for (uint32_t i0w = first; i0w < vocab && !done; i0w += 32 * SAMPLE_THREADS) {
                     const uint32_t i = i0w + lane * SAMPLE_THREADS;
                     float e = 0.0f;
-                    bool live = false;
                     if (i < vocab) {
                         const float xi = x[i];
-                        if (xi > low) { e = soft_exp2(__fmul_rn(__fsub_rn(xi, lmax), c)); live = true; }
+                        if (xi > low) e = soft_exp2(__fmul_rn(__fsub_rn(xi, lmax), c));
                     }
-                    const uint32_t lives = __ballot_sync(0xffffffffu, live);
-                    for (uint32_t l = 0; l < 32 && !done; l++) {
-                        const float el = __shfl_sync(0xffffffffu, e, l);
-                        if (!((lives >> l) & 1u)) continue;
-                        acc = __fadd_rn(acc, el);
-                        if (el > 0.0f) j = i0w + l * SAMPLE_THREADS;
-                        if (rest < acc) done = true;
-                    }
+                    walk_32(e, i0w, rest, acc, j, done);
                 }
                 if (int(lane) == src) pick = j;
             }
@@ -525,7 +517,6 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) sa
     pdl_start();
     if (row_skip && row_skip[blockIdx.x / SC_CTAS]) return;  // the whole cluster leaves: no cluster barrier has been entered
     __shared__ ScExchange xc;
-    __shared__ float vals[SC_THREADS], pre[SC_THREADS], tot_all[32], base[33];
     __shared__ float wbv[SC_WARPS];
     __shared__ uint32_t wbi[SC_WARPS];
     uint32_t rank;
@@ -597,7 +588,7 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) sa
         for (uint32_t i = i0; i < vocab; i += SAMPLE_THREADS) sum = __fadd_rn(sum, soft_exp2(__fmul_rn(__fsub_rn(own(i), lmax), c)));
         float lo, hi, total;
         uint32_t scans = 0;
-        sc_scan(sum, scans++ & 1, &xc, vals, pre, tot_all, base, rank, tid, lo, hi, total);
+        sc_scan(sum, scans++ & 1, &xc, rank, tid, lo, hi, total);
         const float z = total;
         float low = -INFINITY;
         for (uint32_t round = 0; round < SAMPLE_ROUNDS; round++) {
@@ -616,19 +607,11 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) sa
                 for (uint32_t i0w = first; i0w < vocab && !done; i0w += 32 * SAMPLE_THREADS) {
                     const uint32_t i = i0w + lane * SAMPLE_THREADS;
                     float e = 0.0f;
-                    bool live = false;
                     if (i < vocab) {
                         const float xi = STAGED ? sc_row[(i / SAMPLE_THREADS) * SC_THREADS + col] : x[i];
-                        if (xi > low) { e = soft_exp2(__fmul_rn(__fsub_rn(xi, lmax), c)); live = true; }
+                        if (xi > low) e = soft_exp2(__fmul_rn(__fsub_rn(xi, lmax), c));
                     }
-                    const uint32_t lives = __ballot_sync(0xffffffffu, live);
-                    for (uint32_t l = 0; l < 32 && !done; l++) {
-                        const float el = __shfl_sync(0xffffffffu, e, l);
-                        if (!((lives >> l) & 1u)) continue;
-                        acc = __fadd_rn(acc, el);
-                        if (el > 0.0f) j = i0w + l * SAMPLE_THREADS;
-                        if (rest < acc) done = true;
-                    }
+                    walk_32(e, i0w, rest, acc, j, done);
                 }
                 if (int(lane) == src) xc.pick[pb] = j;
             }
@@ -660,7 +643,7 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) sa
                 const float xi = own(i);
                 if (xi > xj) q = __fadd_rn(q, soft_exp2(__fmul_rn(__fsub_rn(xi, lmax), c)));
             }
-            sc_scan(q, scans++ & 1, &xc, vals, pre, tot_all, base, rank, tid, lo, hi, total);
+            sc_scan(q, scans++ & 1, &xc, rank, tid, lo, hi, total);
             if (total < __fmul_rn(row.top_p, z)) { tok = j; break; }
             low = xj;
         }

@@ -10,9 +10,8 @@
 //   at the first rejected i the replacement is drawn from max(0, ep_j Zq - eq_j Zp) by the sampler's
 //   inverse CDF at uniform01(seed, pos0 + i, 1); with all accepted, the bonus token from p_k at
 //   uniform01(seed, pos0 + k, 0). Outputs: accepted count, that token, rollback = k - accepted.
-// Two kernels: per-row statistics (max, argmax, Z) for all S (2k + 1) rows at once -- one pass
-// over the logits from HBM -- then a cluster of 8 blocks per stream that decides and draws (its two rows
-// come from L2).
+// Two kernels: statistics for all S (2k + 1) rows at once, a cluster of 8 blocks a row and one read of the logits, then a
+// cluster of 8 blocks per stream that decides and draws (its two rows come from L2).
 #include <cfloat>
 #include <cmath>
 #include <mutex>
@@ -57,49 +56,160 @@ __device__ void tg_scan(float v, float* ex, float* base, uint32_t tid) {
 
 using vlt::SpecRowStats;
 typedef SpecRowStats RowStats;
+typedef vlt::SpecRowWork RowWork;
 
 __device__ __forceinline__ float e_of(uint16_t x, float mx, float c) { return soft_exp2(__fmul_rn(__fsub_rn(bf16_to_f32(x), mx), c)); }
+// e(x) for two logits that are at most mx (or NaN): soft_exp2_scaled_x2 without what only a positive exponent needs, and
+// with the exponent's bits shifted straight out of the rounding constant's sum (its own bits fall out at the top). The same
+// operations on the value, so the same bits.
+__device__ __forceinline__ float2 e_below_x2(float x0, float x1, float minus_mx, float c) {
+    const float2 x = __fmul2_rn(__fadd2_rn(make_float2(x0, x1), make_float2(minus_mx, minus_mx)), make_float2(c, c));
+    const float2 t = __fadd2_rn(x, make_float2(12582912.0f, 12582912.0f));
+    const float2 f = __ffma2_rn(__fadd2_rn(t, make_float2(-12582912.0f, -12582912.0f)), make_float2(-1.0f, -1.0f), x);
+    float2 p = make_float2(0.00015403530393381608f, 0.00015403530393381608f);
+    p = __ffma2_rn(p, f, make_float2(0.0013333558146428443f, 0.0013333558146428443f));
+    p = __ffma2_rn(p, f, make_float2(0.009618129107628477f, 0.009618129107628477f));
+    p = __ffma2_rn(p, f, make_float2(0.05550410866482158f, 0.05550410866482158f));
+    p = __ffma2_rn(p, f, make_float2(0.2402265069591007f, 0.2402265069591007f));
+    p = __ffma2_rn(p, f, make_float2(0.6931471805599453f, 0.6931471805599453f));
+    p = __ffma2_rn(p, f, make_float2(1.0f, 1.0f));
+    return make_float2(x.x > -125.5f ? __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)) : 0.0f,
+                       x.y > -125.5f ? __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)) : 0.0f);
+}
+// The larger of two bf16 each (the number where one is a NaN).
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
 
-// One block per row of logits (p rows first, then q rows): max, argmax (ties to the lowest id), Z.
-__global__ void __launch_bounds__(THREADS) stats_kernel(const uint16_t* __restrict__ p, const uint16_t* __restrict__ q, uint32_t p_rows, uint32_t vocab,
-                                                        float c, RowStats* out) {
-    __shared__ float ex[THREADS + THREADS / 32 + 1];
-    __shared__ float base[32];
-    __shared__ float bvs[32];
-    __shared__ uint32_t bis[32];
-    const uint32_t r = blockIdx.x, tid = threadIdx.x, lane = tid % 32;
-    const uint16_t* x = r < p_rows ? p + size_t(r) * vocab : q + size_t(r - p_rows) * vocab;
-    float mx = -FLT_MAX;
-    uint32_t am = 0xffffffffu;
-    {
-        uint32_t i0 = tid;
-        for (; i0 + 7 * THREADS < vocab; i0 += 8 * THREADS) {
+// A block's share of a row -- 128 ids of every 1024: of the 1024 "threads" of the sampler's order the cluster's 8 x 128 -- in
+// shared memory: [id / 1024][128]. `vec`: rows start on 16-byte boundaries and hold whole groups of 8 ids, so that the
+// share comes by 16-byte asynchronous copies, all in flight at once; else two bytes at a time. N: the block's threads.
+constexpr size_t STAGE_MAX = 100 * 1024;  // of one row's share; longer rows are read from global memory at every pass
+__host__ __device__ constexpr uint32_t stage_chunks(uint32_t vocab) { return (vocab + THREADS - 1) / THREADS; }
+__host__ __device__ constexpr size_t stage_bytes(uint32_t vocab) { return size_t(stage_chunks(vocab)) * SC_THREADS * 2; }
+template <uint32_t N>
+__device__ __forceinline__ void stage_row(const uint16_t* x, uint32_t vocab, bool vec, uint16_t* sm, uint32_t rank, uint32_t tid) {
+    const uint32_t chunks = stage_chunks(vocab);
+    if (vec) {
+        const uint32_t dst = uint32_t(__cvta_generic_to_shared(sm));
+        for (uint32_t g = tid; g < chunks * (SC_THREADS / 8); g += N) {
+            const uint32_t id = g / (SC_THREADS / 8) * THREADS + rank * SC_THREADS + g % (SC_THREADS / 8) * 8;
+            if (id < vocab) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + g * 16), "l"(x + id) : "memory");
+        }
+        return;
+    }
+    for (uint32_t i = tid; i < SC_THREADS; i += N) {
+        const uint32_t first = rank * SC_THREADS + i, n = vocab - min(vocab, first);  // ids from this column's first on
+        uint32_t ch = 0;
+        for (; ch + 7 < chunks && (ch + 7) * THREADS < n; ch += 8) {
             uint16_t v[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = x[i0 + u * THREADS];
+            for (int u = 0; u < 8; u++) v[u] = x[first + (ch + u) * THREADS];
 #pragma unroll
-            for (int u = 0; u < 8; u++) better(mx, am, bf16_to_f32(v[u]), i0 + u * THREADS);
+            for (int u = 0; u < 8; u++) sm[(ch + u) * SC_THREADS + i] = v[u];
         }
-        for (; i0 < vocab; i0 += THREADS) better(mx, am, bf16_to_f32(x[i0]), i0);
+        for (; ch * THREADS < n; ch++) sm[ch * SC_THREADS + i] = x[first + ch * THREADS];
     }
-    warp_best(mx, am);
-    if (lane == 0) { bvs[tid / 32] = mx; bis[tid / 32] = am; }
+}
+__device__ __forceinline__ void stage_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    mx = bvs[0];
-    am = bis[0];
-    for (uint32_t i = 1; i < 32; i++) better(mx, am, bvs[i], bis[i]);
-    float s = 0.0f;
-    uint32_t i0 = tid;
-    for (; i0 + 7 * THREADS < vocab; i0 += 8 * THREADS) {  // eight loads in flight, the additions in id order
-        uint16_t v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = x[i0 + u * THREADS];
-#pragma unroll
-        for (int u = 0; u < 8; u++) s = __fadd_rn(s, e_of(v[u], mx, c));
+}
+
+__device__ __forceinline__ float row_max(const RowWork& w) {
+    const float4 a = *reinterpret_cast<const float4*>(w.max), b = *reinterpret_cast<const float4*>(w.max + 4);
+    return fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+}
+
+// A cluster of 8 blocks per row of logits (p rows first, then q rows): each block's best logit with the lowest id it has
+// there, and the sums of e over the row in the sampler's order (thread t of 1024: ids t, t + 1024, ...) as the totals of its
+// 32 groups of 32 threads; with a q row its draft id, read here once (an id past the vocabulary as 0, see
+// launch_spec_accept_static). The row is read from memory once. A thread stands for two neighbours of the 1024, whose sums
+// are the halves of packed registers; the maximum is taken on packed bf16, whoever's ids they are. What the cluster has to
+// agree on is the maximum alone: every block stores its own into the others and there is one barrier.
+// What bounds it: a row's 256 KiB of shared memory let 131 rows run at a time, and such a wave takes 5 us of HBM, 5 us of the
+// fp32 pipe (11 packed operations for two ids) and a barrier one after another. Three kernels without clusters that read the
+// row twice (maxima; sums; decision) took 24 / 67 us with the decision at 18 / 288 rows of 128 256 ids, one block per row
+// 73 / 122, this 21 / 62.
+constexpr uint32_t STATS_THREADS = SC_THREADS / 2;
+template <bool STAGED>
+__global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(STATS_THREADS) stats_kernel(const uint16_t* __restrict__ p, const uint16_t* __restrict__ q,
+                                                                                           const uint32_t* __restrict__ drafts, uint32_t p_rows, uint32_t vocab, bool vec,
+                                                                                           float c, RowWork* work) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ __align__(16) uint16_t row_sm[];
+    __shared__ float maxima[SC_CTAS];
+    __shared__ uint32_t wbv[STATS_THREADS / 32], first_id;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const uint32_t r = blockIdx.x / SC_CTAS, tid = threadIdx.x, lane = tid % 32, vt = rank * SC_THREADS + 2 * tid;  // and vt + 1
+    const uint16_t* x = r < p_rows ? p + size_t(r) * vocab : q + size_t(r - p_rows) * vocab;
+    const uint32_t chunks = stage_chunks(vocab);
+    uint32_t draft = 0;
+    if (tid == 0) {
+        first_id = 0xffffffffu;
+        if (rank == 0 && r >= p_rows) draft = drafts[r - p_rows];
     }
-    for (; i0 < vocab; i0 += THREADS) s = __fadd_rn(s, e_of(x[i0], mx, c));
-    tg_scan(s, ex, base, tid);
-    if (tid == 0) out[r] = RowStats{mx, am, ex[ex_at(THREADS)], 0};
+    if (STAGED) {
+        stage_row<STATS_THREADS>(x, vocab, vec, row_sm, rank, tid);
+        // What the last 1024 ids lack stands as -inf, whose e is 0.
+        for (uint32_t i = tid; i < SC_THREADS; i += STATS_THREADS)
+            if ((chunks - 1) * THREADS + rank * SC_THREADS + i >= vocab) row_sm[(chunks - 1) * SC_THREADS + i] = 0xff80u;
+        stage_wait();
+    }
+    auto pair_at = [&](uint32_t ch) {
+        if (STAGED) return reinterpret_cast<const uint32_t*>(row_sm)[ch * (SC_THREADS / 2) + tid];
+        const uint32_t i = ch * THREADS + vt;
+        return (i < vocab ? uint32_t(x[i]) : 0xff80u) | (i + 1 < vocab ? uint32_t(x[i + 1]) << 16 : 0xff800000u);
+    };
+    uint32_t best = 0xff80ff80u;
+#pragma unroll 8
+    for (uint32_t ch = 0; ch < chunks; ch++) best = max_bf16x2(best, pair_at(ch));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max_bf16x2(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (lane == 0) wbv[tid / 32] = best;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t w = 0; w < STATS_THREADS / 32; w++) best = max_bf16x2(best, wbv[w]);
+    const float mine = fmaxf(-FLT_MAX, fmaxf(bf16lo(best), bf16hi(best)));
+    if (tid < SC_CTAS) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sc_remote(&maxima[rank], tid)), "f"(mine) : "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    {  // meanwhile the lowest id of the share's own best
+        uint32_t id = 0xffffffffu;
+#pragma unroll 8
+        for (uint32_t ch = 0; ch < chunks; ch++) {
+            const uint32_t v = pair_at(ch), i = ch * THREADS + vt;
+            id = min(id, bf16lo(v) == mine ? i : bf16hi(v) == mine ? i + 1 : 0xffffffffu);
+        }
+        id = __reduce_min_sync(0xffffffffu, id);
+        if (lane == 0) atomicMin(&first_id, id);
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // (of the block's threads too; no block touches another's memory after it)
+    float mx = maxima[0];
+#pragma unroll
+    for (uint32_t s = 1; s < SC_CTAS; s++) mx = fmaxf(mx, maxima[s]);
+    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll 8
+    for (uint32_t ch = 0; ch < chunks; ch++) {
+        const uint32_t v = pair_at(ch);
+        sum = __fadd2_rn(sum, e_below_x2(bf16lo(v), bf16hi(v), -mx, c));
+    }
+    // A group of 32 of the 1024 is half a warp: its sums left to right.
+    float group = 0.0f;
+#pragma unroll
+    for (uint32_t l = 0; l < 16; l++) {
+        group = __fadd_rn(group, __shfl_sync(0xffffffffu, sum.x, l, 16));
+        group = __fadd_rn(group, __shfl_sync(0xffffffffu, sum.y, l, 16));
+    }
+    if (lane % 16 == 0) work[r].tot[rank * SC_WARPS + tid / 16] = group;
+    __syncthreads();
+    if (tid == 0) {
+        work[r].max[rank] = mine;
+        work[r].argmax[rank] = first_id;
+        if (rank == 0) work[r].draft = draft < vocab ? draft : 0u;
+    }
 }
 
 // The sampler's inverse CDF (kernels.metal:1540-1559) over weights w(i) >= 0; `fallback` if they
@@ -129,14 +239,7 @@ __device__ uint32_t inverse_cdf(uint32_t vocab, W w, float u, uint32_t fallback,
         bool done = false;
         for (uint32_t i0 = first; i0 < vocab && !done; i0 += 32 * THREADS) {
             const uint32_t i = i0 + lane * THREADS;
-            const float e = i < vocab ? w(i) : 0.0f;
-            const uint32_t n_live = min(32u, (vocab - i0 + THREADS - 1) / THREADS);
-            for (uint32_t l = 0; l < n_live && !done; l++) {
-                const float el = __shfl_sync(0xffffffffu, e, l);
-                acc = __fadd_rn(acc, el);
-                if (el > 0.0f) j = i0 + l * THREADS;
-                if (rest < acc) done = true;
-            }
+            walk_32(i < vocab ? w(i) : 0.0f, i0, rest, acc, j, done);
         }
         if (int(lane) == src) *pick = j;
     }
@@ -147,54 +250,117 @@ __device__ uint32_t inverse_cdf(uint32_t vocab, W w, float u, uint32_t fallback,
 
 // The decision, a cluster of 8 blocks per stream: the 1024 "threads" of the sampler's order are the cluster's 8 x 128 (as
 // in the sampler's cluster form), so every sum keeps its order and association while a stream's pass over its two rows
-// runs on eight SMs (one block per stream left 116 of 148 SMs idle at 32 streams).
+// runs on eight SMs. Every block first finishes the rows' sums, a warp a row, and runs the tests, a lane each, so that
+// their chains of loads run side by side. Bound by latency; the rows' shares are staged as above, and the pass that adds up
+// and the walk to the token read them there (an id at a time from L2, they took 90 us).
+constexpr uint32_t MAX_ROWS = 31;  // 2 k + 1 at most
+template <bool STAGED>
 __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) decide_cluster_kernel(const uint16_t* __restrict__ p, const uint16_t* __restrict__ q,
-                                                                                                 const uint32_t* __restrict__ drafts, const RowStats* __restrict__ stats,
-                                                                                                 uint32_t streams, uint32_t k, uint32_t vocab, float c,
-                                                                                                 const uint64_t* __restrict__ seeds, const uint32_t* __restrict__ pos0,
-                                                                                                 uint32_t* accepted, uint32_t* token, uint32_t* rollback) {
+                                                                                                 const RowWork* __restrict__ work, uint32_t streams, uint32_t k,
+                                                                                                 uint32_t vocab, bool vec, float c, const uint64_t* __restrict__ seeds,
+                                                                                                 const uint32_t* __restrict__ pos0, uint32_t* accepted, uint32_t* token,
+                                                                                                 uint32_t* rollback) {
+    pdl_start();
+    extern __shared__ __align__(16) uint16_t row_sm[];  // p's share, then q's
     __shared__ ScExchange xc;
-    __shared__ float vals[SC_THREADS], pre[SC_THREADS], tot_all[32], base[33];
+    __shared__ float z_s[MAX_ROWS], max_s[MAX_ROWS];  // the k + 1 p rows, then the k q rows
     __shared__ uint32_t first_reject;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    const uint32_t s = blockIdx.x / SC_CTAS, tid = threadIdx.x;
-    const uint32_t seed_lo = uint32_t(seeds[s]), seed_hi = uint32_t(seeds[s] >> 32);
-    const RowStats* ps = stats + size_t(s) * (k + 1);
-    const RowStats* qs = stats + size_t(streams) * (k + 1) + size_t(s) * k;
+    const uint32_t s = blockIdx.x / SC_CTAS, tid = threadIdx.x, lane = tid % 32, vt = rank * SC_THREADS + tid;
+    const uint64_t seed = seeds[s];
+    const uint32_t seed_lo = uint32_t(seed), seed_hi = uint32_t(seed >> 32), first_pos = pos0[s];
+    const RowWork* pw = work + size_t(s) * (k + 1);
+    const RowWork* qw = work + size_t(streams) * (k + 1) + size_t(s) * k;
     const uint16_t* pp = p + size_t(s) * (k + 1) * vocab;
     const uint16_t* qq = q + size_t(s) * k * vocab;
-    if (tid == 0) {  // every block runs the few tests itself: cheaper than sending the result round
-        uint32_t i = 0;
-        for (; i < k; i++) {
-            const uint32_t x = drafts[s * k + i];
-            const float ep = e_of(pp[size_t(i) * vocab + x], ps[i].max, c), eq = e_of(qq[size_t(i) * vocab + x], qs[i].max, c);
-            const float u = uniform01(seed_lo, seed_hi, pos0[s] + i, 0);
-            const float lhs = __fmul_rn(__fmul_rn(u, eq), ps[i].z), rhs = __fmul_rn(ep, qs[i].z);
-            if (!(lhs < rhs)) break;
-        }
-        first_reject = i;
+    uint16_t xp = 0, xq = 0;
+    if (tid < k) {
+        const uint32_t draft = qw[tid].draft;
+        xp = pp[size_t(tid) * vocab + draft];
+        xq = qq[size_t(tid) * vocab + draft];
+    }
+    for (uint32_t r = tid / 32; r < 2 * k + 1; r += SC_WARPS) {
+        const RowWork& w = r <= k ? pw[r] : qw[r - k - 1];
+        const float tot = w.tot[lane], mx = row_max(w);
+        float z;
+        lane_prefix(tot, lane, z);
+        if (lane == 0) { z_s[r] = z; max_s[r] = mx; }
+    }
+    if (tid == 0) {
         xc.pick[0] = 0xffffffffu;
         xc.pick[1] = 0xffffffffu;
     }
     __syncthreads();
+    if (tid < 32) {  // every block runs the few tests itself: cheaper than sending the result round
+        bool fails = false;  // a lane without a test does not fail
+        if (tid < k) {
+            const float ep = e_of(xp, max_s[tid], c), eq = e_of(xq, max_s[k + 1 + tid], c);
+            const float u = uniform01(seed_lo, seed_hi, first_pos + tid, 0);
+            const float lhs = __fmul_rn(__fmul_rn(u, eq), z_s[tid]), rhs = __fmul_rn(ep, z_s[k + 1 + tid]);
+            fails = !(lhs < rhs);
+        }
+        const uint32_t failed = __ballot_sync(0xffffffffu, fails);
+        if (tid == 0) first_reject = failed ? uint32_t(__ffs(failed) - 1) : k;
+    }
+    __syncthreads();
     const uint32_t i = first_reject;
-    uint32_t tok;
-    if (i < k) {
-        const uint16_t* pi = pp + size_t(i) * vocab;
-        const uint16_t* qi = qq + size_t(i) * vocab;
-        const float pm = ps[i].max, qm = qs[i].max, zp = ps[i].z, zq = qs[i].z;
+    const bool rejected = i < k;
+    const uint16_t* pi = pp + size_t(i) * vocab;
+    const uint16_t* qi = qq + size_t(rejected ? i : 0) * vocab;
+    uint16_t* q_sm = row_sm + stage_chunks(vocab) * SC_THREADS;
+    if (STAGED) {
+        stage_row<SC_THREADS>(pi, vocab, vec, row_sm, rank, tid);
+        if (rejected) stage_row<SC_THREADS>(qi, vocab, vec, q_sm, rank, tid);
+    }
+    // The token if the weights sum to 0 or the target falls past the last of them: p's best, the lowest id of them.
+    float best = -FLT_MAX;
+    uint32_t fallback = 0xffffffffu;
+#pragma unroll
+    for (uint32_t sl = 0; sl < SPEC_SLICES; sl++) better(best, fallback, pw[i].max[sl], pw[i].argmax[sl]);
+    if (STAGED) stage_wait();
+    auto at = [&](const uint16_t* x, const uint16_t* sm, uint32_t j) { return STAGED ? sm[j / THREADS * SC_THREADS + j % SC_THREADS] : x[j]; };  // ids of this block's share
+    constexpr uint32_t B = 8;
+    uint32_t tok, i0 = vt;
+    float a = 0.0f;
+    if (rejected) {
+        const float pm = max_s[i], qm = max_s[k + 1 + i], zp = z_s[i], zq = z_s[k + 1 + i];
         auto resid = [&](uint32_t j) {
-            const float a = __fmul_rn(e_of(pi[j], pm, c), zq), b = __fmul_rn(e_of(qi[j], qm, c), zp);
-            const float d = __fsub_rn(a, b);
+            const float ea = __fmul_rn(e_of(at(pi, row_sm, j), pm, c), zq), eb = __fmul_rn(e_of(at(qi, q_sm, j), qm, c), zp);
+            const float d = __fsub_rn(ea, eb);
             return d > 0.0f ? d : 0.0f;
         };
-        tok = sc_inverse_cdf(vocab, resid, uniform01(seed_lo, seed_hi, pos0[s] + i, 1), ps[i].argmax, &xc, 0, 0, vals, pre, tot_all, base, rank, tid);
+        for (; i0 + (B - 1) * THREADS < vocab; i0 += B * THREADS) {
+            float vp[B], vq[B];
+#pragma unroll
+            for (uint32_t u = 0; u < B; u++) {
+                vp[u] = bf16_to_f32(at(pi, row_sm, i0 + u * THREADS));
+                vq[u] = bf16_to_f32(at(qi, q_sm, i0 + u * THREADS));
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < B; u += 2) {
+                const float2 ea = __fmul2_rn(e_below_x2(vp[u], vp[u + 1], -pm, c), make_float2(zq, zq));
+                const float2 eb = __fmul2_rn(e_below_x2(vq[u], vq[u + 1], -qm, c), make_float2(zp, zp));
+                const float d0 = __fsub_rn(ea.x, eb.x), d1 = __fsub_rn(ea.y, eb.y);
+                a = __fadd_rn(a, d0 > 0.0f ? d0 : 0.0f);
+                a = __fadd_rn(a, d1 > 0.0f ? d1 : 0.0f);
+            }
+        }
+        tok = sc_inverse_cdf_rest(vocab, resid, a, i0, uniform01(seed_lo, seed_hi, first_pos + i, 1), fallback, &xc, 0, 0, rank, tid);
     } else {
-        const uint16_t* pk = pp + size_t(k) * vocab;
-        const float pm = ps[k].max;
-        auto w = [&](uint32_t j) { return e_of(pk[j], pm, c); };
-        tok = sc_inverse_cdf(vocab, w, uniform01(seed_lo, seed_hi, pos0[s] + k, 0), ps[k].argmax, &xc, 0, 0, vals, pre, tot_all, base, rank, tid);
+        const float pm = max_s[k];
+        auto w = [&](uint32_t j) { return e_of(at(pi, row_sm, j), pm, c); };
+        for (; i0 + (B - 1) * THREADS < vocab; i0 += B * THREADS) {
+            float v[B];
+#pragma unroll
+            for (uint32_t u = 0; u < B; u++) v[u] = bf16_to_f32(at(pi, row_sm, i0 + u * THREADS));
+#pragma unroll
+            for (uint32_t u = 0; u < B; u += 2) {
+                const float2 e = e_below_x2(v[u], v[u + 1], -pm, c);
+                a = __fadd_rn(__fadd_rn(a, e.x), e.y);
+            }
+        }
+        tok = sc_inverse_cdf_rest(vocab, w, a, i0, uniform01(seed_lo, seed_hi, first_pos + k, 0), fallback, &xc, 0, 0, rank, tid);
     }
     if (rank == 0 && tid == 0) {
         accepted[s] = i;
@@ -206,15 +372,42 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) de
 
 }  // namespace spec
 
-// p [S][k+1][V], q [S][k][V] bf16 on the device; stats: scratch for S (2k + 1) rows of 16 bytes.
-void launch_spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t* drafts, uint32_t streams, uint32_t k, uint32_t vocab, float temperature,
-                        const uint64_t* seeds, const uint32_t* pos0, void* stats, uint32_t* accepted, uint32_t* token, uint32_t* rollback, cudaStream_t s) {
+// p [S][k+1][V], q [S][k][V] bf16 on the device; work: scratch for S (2k + 1) rows. The first kernel overlaps with nothing
+// before it (the caller's stream may hold anything); the second's launch overlaps with it.
+// Returns the first error of the launches.
+cudaError_t launch_spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t* drafts, uint32_t streams, uint32_t k, uint32_t vocab, float temperature,
+                               const uint64_t* seeds, const uint32_t* pos0, SpecRowWork* work, uint32_t* accepted, uint32_t* token, uint32_t* rollback, cudaStream_t s) {
+    using namespace spec;
     const float c = LOG2E / temperature;  // the same IEEE division as the device's __fdiv_rn
-    spec::stats_kernel<<<streams * (2 * k + 1), spec::THREADS, 0, s>>>(p, q, streams * (k + 1), vocab, c, static_cast<spec::RowStats*>(stats));
+    const size_t share = stage_bytes(vocab);
+    const bool staged = share <= STAGE_MAX, vec = vocab % 8 == 0 && (reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(q)) % 16 == 0;
+    static PerDevice configured;
+    cudaError_t e = cudaSuccess;
+    configured.once([&] {
+        e = cudaFuncSetAttribute(stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(STAGE_MAX));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(decide_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(2 * STAGE_MAX));
+    });
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = s;
+    cfg.blockDim = dim3(STATS_THREADS);
+    cfg.gridDim = dim3(streams * (2 * k + 1) * SC_CTAS);
+    cfg.dynamicSmemBytes = staged ? share : 0;
+    e = cudaLaunchKernelEx(&cfg, staged ? stats_kernel<true> : stats_kernel<false>, p, q, drafts, streams * (k + 1), vocab, vec, c, work);
+    if (e != cudaSuccess) return e;
     launch_counter()++;
-    spec::decide_cluster_kernel<<<streams * SC_CTAS, SC_THREADS, 0, s>>>(p, q, drafts, static_cast<const spec::RowStats*>(stats), streams, k, vocab, c, seeds, pos0,
-                                                                        accepted, token, rollback);
-    launch_counter()++;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.gridDim = dim3(streams * SC_CTAS);
+    cfg.dynamicSmemBytes = staged ? 2 * share : 0;
+    e = cudaLaunchKernelEx(&cfg, staged ? decide_cluster_kernel<true> : decide_cluster_kernel<false>, p, q, static_cast<const RowWork*>(work), streams, k, vocab, vec, c, seeds, pos0,
+                           accepted, token, rollback);
+    if (e == cudaSuccess) launch_counter()++;
+    return e;
 }
 
 // ------------------------------------------------ the rule inside the engine's step
@@ -301,7 +494,6 @@ __global__ void __launch_bounds__(THREADS) step_stats_kernel(const SpecStepArgs 
 __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) step_decide_kernel(const SpecStepArgs a) {
     pdl_start();
     __shared__ ScExchange xc;
-    __shared__ float vals[SC_THREADS], pre[SC_THREADS], tot_all[32], base[33];
     __shared__ uint32_t first_reject;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -377,13 +569,13 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(SC_THREADS) st
                 e[u] = d > 0.0f ? d : 0.0f;
             }
         };
-        tok = sc_inverse_cdf_batched<B>(a.vocab, resid, resid_batch, uniform01(sr.seed_lo, sr.seed_hi, a.meta[2 * (ru.first + i) + 1], 1), ps[i - 1].argmax, &xc, 0, 0, vals, pre,
-                                        tot_all, base, rank, tid);
+        tok = sc_inverse_cdf_batched<B>(a.vocab, resid, resid_batch, uniform01(sr.seed_lo, sr.seed_hi, a.meta[2 * (ru.first + i) + 1], 1), ps[i - 1].argmax, &xc, 0, 0,
+                                        rank, tid);
     } else {
         const float* pk = pp + size_t(ru.count - 1) * a.vocab;
         const float pm = ps[ru.count - 1].max;
         auto w = [&](uint32_t j) { return e_of(pk[j], pm); };
-        tok = sc_inverse_cdf<16>(a.vocab, w, uniform01(sr.seed_lo, sr.seed_hi, a.meta[2 * (ru.first + ru.count - 1) + 1] + 1, 0), ps[ru.count - 1].argmax, &xc, 0, 0, vals, pre, tot_all, base, rank, tid);
+        tok = sc_inverse_cdf<16>(a.vocab, w, uniform01(sr.seed_lo, sr.seed_hi, a.meta[2 * (ru.first + ru.count - 1) + 1] + 1, 0), ps[ru.count - 1].argmax, &xc, 0, 0, rank, tid);
     }
     if (rank == 0 && tid == 0) {
         for (uint32_t j = 0; j + 1 < i; j++) a.out[ru.head0 + j] = a.tokens[ru.first + j + 1];
@@ -455,46 +647,29 @@ void launch_draft_draw(const float* logits, uint32_t v, const uint32_t* vocab_id
 // A variant for callers that cannot allocate device memory when they need an acceptance step:
 // a serving loop that has handed every byte of the device to its own pools, or one that must not
 // pay the device-wide synchronisation an allocation or a free can imply in the middle of decoding.
-// Its scratch (the per-row statistics, and a bounds-checked copy of the draft ids) lives in
-// file-scope device arrays of a fixed size, so a step may cover at most STATIC_MAX_ROWS rows of
-// logits. The arrays' addresses are looked up once per device, on the first call made with that
-// device current; that first call is set-up and belongs before the caller starts any stream
-// capture. All calls on a device share the arrays: nothing in them has to start at zero (the first
-// kernel overwrites every word the later ones read), but two calls in flight at once on one
-// device race on them.
+// Its scratch (the rows' statistics and bounds-checked draft ids) lives in a file-scope device
+// array of a fixed size, so a step may cover at most STATIC_MAX_ROWS rows of logits. The array's
+// address is looked up once per device, on the first call made with that device current; that
+// first call is set-up and belongs before the caller starts any stream capture. All calls on a
+// device share the array: nothing in it has to start at zero (the first kernel overwrites every
+// word the second reads), but two calls in flight at once on one device race on it.
 namespace spec {
 
 constexpr uint32_t STATIC_MAX_ROWS = 2048;  // streams * (2 k + 1) rows of logits a call may cover
-static __device__ __align__(256) RowStats static_stats[STATIC_MAX_ROWS];
-static __device__ __align__(256) uint32_t static_drafts[STATIC_MAX_ROWS];
+static __device__ __align__(256) RowWork static_work[STATIC_MAX_ROWS];
 
-// The caller's draft ids cannot be checked on the host here; an id past the vocabulary is read as 0
-// instead of indexing out of the logits (that stream's result then means nothing).
-__global__ void copy_drafts_kernel(const uint32_t* __restrict__ drafts, uint32_t n, uint32_t vocab, uint32_t* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = drafts[i] < vocab ? drafts[i] : 0u;
-}
-
-struct StaticScratch {
-    RowStats* stats;
-    uint32_t* drafts;
-};
-
-// The arrays' addresses on the current device; looked up (cudaGetSymbolAddress) on the first call per device.
-static const char* static_scratch(StaticScratch* out) {
+// The array's address on the current device; looked up (cudaGetSymbolAddress) on the first call per device.
+static const char* static_scratch(RowWork** out) {
     constexpr int MAX_DEVICES = 64;
-    static StaticScratch table[MAX_DEVICES] = {};
+    static RowWork* table[MAX_DEVICES] = {};
     static std::mutex mu;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return "spec_accept_static: no usable current device";
     std::lock_guard<std::mutex> lock(mu);
-    if (!table[dev].stats) {
+    if (!table[dev]) {
         void* ps = nullptr;
-        void* pd = nullptr;
-        if (cudaGetSymbolAddress(&ps, static_stats) != cudaSuccess || !ps) return "spec_accept_static: cudaGetSymbolAddress failed for the statistics array";
-        if (cudaGetSymbolAddress(&pd, static_drafts) != cudaSuccess || !pd) return "spec_accept_static: cudaGetSymbolAddress failed for the draft array";
-        table[dev].drafts = static_cast<uint32_t*>(pd);
-        table[dev].stats = static_cast<RowStats*>(ps);
+        if (cudaGetSymbolAddress(&ps, static_work) != cudaSuccess || !ps) return "spec_accept_static: cudaGetSymbolAddress failed for the scratch array";
+        table[dev] = static_cast<RowWork*>(ps);
     }
     *out = table[dev];
     return nullptr;
@@ -514,13 +689,12 @@ const char* launch_spec_accept_static(const uint16_t* p, const uint16_t* q, cons
     if (!(std::isnormal(temperature) && temperature > 0.0f)) return "spec_accept_static: needs a normal positive temperature";
     if (uint64_t(streams) * (2 * k + 1) > spec::STATIC_MAX_ROWS)
         return "spec_accept_static: streams * (2 k + 1) exceeds the 2048 rows the static scratch holds; use vlt_spec_accept";
-    spec::StaticScratch sc{};
-    if (const char* e = spec::static_scratch(&sc)) return e;
-    const uint32_t n = streams * k;
-    spec::copy_drafts_kernel<<<(n + 255) / 256, 256, 0, s>>>(drafts, n, vocab, sc.drafts);
-    launch_counter()++;
-    launch_spec_accept(p, q, sc.drafts, streams, k, vocab, temperature, seeds, pos0, sc.stats, accepted, token, rollback, s);
-    return cudaGetLastError() == cudaSuccess ? nullptr : "spec_accept_static: kernel launch failed";
+    // The caller's draft ids cannot be checked on the host here; an id past the vocabulary is read as 0 instead of
+    // indexing out of the logits (that stream's result then means nothing).
+    spec::RowWork* work = nullptr;
+    if (const char* e = spec::static_scratch(&work)) return e;
+    const cudaError_t e = launch_spec_accept(p, q, drafts, streams, k, vocab, temperature, seeds, pos0, work, accepted, token, rollback, s);
+    return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? nullptr : "spec_accept_static: kernel launch failed";
 }
 
 }  // namespace vlt

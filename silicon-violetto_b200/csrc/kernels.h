@@ -592,6 +592,15 @@ struct SpecRowStats {
     float z;
     uint32_t pad;
 };
+// The stand-alone rule's scratch for a row of logits: maxima and their ids by eighths of the row, the sums of the sampler's 32
+// groups of threads, and a q row's draft.
+constexpr uint32_t SPEC_SLICES = 8;
+struct alignas(16) SpecRowWork {
+    float max[SPEC_SLICES];
+    uint32_t argmax[SPEC_SLICES];
+    float tot[32];
+    uint32_t draft;
+};
 // The rule inside the engine's step (k_spec.cu), device pointers throughout.
 struct SpecStepArgs {
     const RunIn* runs;
@@ -618,8 +627,8 @@ void launch_draft_draw(const float* logits, uint32_t v, const uint32_t* vocab_id
                        const uint32_t* lens, uint32_t n_runs, uint32_t i, uint32_t rule, uint32_t* feed, uint32_t* tree, float* q_keep, uint32_t* q_rows,
                        cudaStream_t s);
 // Rejection-sampling acceptance over bf16 draft and target logits on the device (k_spec.cu).
-void launch_spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t* drafts, uint32_t streams, uint32_t k, uint32_t vocab, float temperature,
-                        const uint64_t* seeds, const uint32_t* pos0, void* stats, uint32_t* accepted, uint32_t* token, uint32_t* rollback, cudaStream_t s);
+cudaError_t launch_spec_accept(const uint16_t* p, const uint16_t* q, const uint32_t* drafts, uint32_t streams, uint32_t k, uint32_t vocab, float temperature,
+                               const uint64_t* seeds, const uint32_t* pos0, SpecRowWork* work, uint32_t* accepted, uint32_t* token, uint32_t* rollback, cudaStream_t s);
 // The same with its scratch in static device arrays: allocates nothing; device pointers throughout.
 // Returns NULL or an error message (a literal).
 uint32_t spec_accept_static_max_rows();
