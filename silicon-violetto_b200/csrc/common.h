@@ -124,6 +124,7 @@ struct Buffer {
         } else {
             VLT_CUDA(cudaMalloc(&dev, n));
             VLT_CUDA(cudaMemset(dev, 0, n));
+            VLT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // cudaMemset may return before it has run, and the engine's own stream does not wait for it: a write queued there could be zeroed again
         }
     }
     void release() {
