@@ -8,8 +8,11 @@
 // 16 rows), walks the keys in blocks of 64 (four pages of K and of V by TMA into a three-stage ring of 128-byte-swizzled
 // shared memory, shared by the four warps; the G heads of a kv head find the same pages in L2), and keeps the whole
 // softmax online in registers: S = Q K^T lands in the accumulator layout that is the A-fragment layout of the next
-// product, so P goes into O += P V without leaving the registers. No key split (a chunk has rows enough to fill the
-// GPU), so no partials and no merge kernel: the block writes the normalised rows, fp32 and bf16.
+// product, so P goes into O += P V without leaving the registers. Two such groups of warps hold the same rows and take the
+// key blocks in turn, each with a ring of its own, and add up in shared memory at the end: a portion of 512 rows is 256
+// blocks, 1.7 an SM, and with four warps each the dependent chain of a key block was what the SM waited on. Two blocks of
+// eight warps still share an SM (128 registers, 97 KB). No partials and no merge kernel: the block writes the normalised
+// rows, fp32 and bf16.
 //
 // The step's own rows are in the cache already (the qkv projection's epilogue wrote them), so every key is read from
 // there; what a row may see is the decode kernel's rule, per row: every cached key below the first position of its
@@ -25,7 +28,7 @@ namespace vlt {
 
 namespace prefill {
 
-constexpr uint32_t CQ = 64, CK = 64, HD = 64, PAGE = 16, WARPS = 4, STAGES = 3;
+constexpr uint32_t CQ = 64, CK = 64, HD = 64, PAGE = 16, WARPS = 4, GROUPS = 2, STAGES = 3;
 constexpr uint32_t STAGE_BYTES = 2 * CK * HD * 2;  // K block then V block
 constexpr uint32_t SPIN_LIMIT = 1u << 24;
 
@@ -46,16 +49,22 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x
                  "r"(y), "r"(bar)
                  : "memory");
 }
-// grid (chunk tiles, query heads), 128 threads.
-__global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a, const __grid_constant__ AttnMaps maps) {
+__device__ __forceinline__ void group_sync(uint32_t grp) {  // (constant barrier numbers: a variable one would claim all sixteen)
+    if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(WARPS * 32) : "memory");
+}
+// grid (chunk tiles, query heads), GROUPS * 128 threads.
+__global__ void __launch_bounds__(GROUPS * WARPS * 32, 2) attn_chunk_kernel(ChunkAttnArgs a, const __grid_constant__ AttnMaps maps) {
     pdl_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));  // the swizzle is a function of address bits 4..9
-    __shared__ uint64_t bars[STAGES];
-    __shared__ uint32_t fail;
+    __shared__ uint64_t bars_all[GROUPS][STAGES];
+    __shared__ uint32_t fail[GROUPS];
 
     const uint32_t tile = blockIdx.x, h = blockIdx.y, kvh = h / (a.n_heads / a.kv.n_kv);
-    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32, g = lane >> 2, tq = lane & 3;
+    const uint32_t grp = threadIdx.x / (WARPS * 32), tid = threadIdx.x % (WARPS * 32), warp = tid / 32, lane = tid % 32, g = lane >> 2, tq = lane & 3;
+    uint8_t* ring = smem + grp * STAGES * STAGE_BYTES;
+    uint64_t* bars = bars_all[grp];
     const uint32_t t0 = a.ctiles[2 * tile], rows = a.ctiles[2 * tile + 1];
     const uint32_t slot = a.meta[2 * t0];
 
@@ -78,10 +87,10 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) block_end = max(block_end, __shfl_xor_sync(0xffffffffu, block_end, o));
     __shared__ uint32_t ends[WARPS];
-    if (lane == 0) ends[warp] = block_end;
+    if (lane == 0 && grp == 0) ends[warp] = block_end;  // (the groups hold the same rows)
     if (tid == 0) {
         for (uint32_t s = 0; s < STAGES; s++) mbar_init(smem_u32(&bars[s]), 1);
-        fail = 0;
+        fail[grp] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -89,11 +98,12 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
     const uint32_t warp_end = ends[warp];
     block_end = max(max(ends[0], ends[1]), max(ends[2], ends[3]));
     const uint32_t n_blocks = (block_end + CK - 1) / CK;
+    const uint32_t my_blocks = (n_blocks + GROUPS - 1 - grp) / GROUPS;  // this group's: grp, grp + GROUPS, ...
 
     const uint32_t* ptab = a.page_table + size_t(slot) * a.kv.max_pages;
     const uint32_t row_base = a.layer * a.kv.n_pages;
-    auto issue = [&](uint32_t b) {  // thread 0: key block b into stage b % STAGES
-        const uint32_t st = b % STAGES, bar = smem_u32(&bars[st]), dst = smem_u32(smem + st * STAGE_BYTES);
+    auto issue = [&](uint32_t i) {  // the group's thread 0: its i-th key block into stage i % STAGES
+        const uint32_t b = i * GROUPS + grp, st = i % STAGES, bar = smem_u32(&bars[st]), dst = smem_u32(ring + st * STAGE_BYTES);
         mbar_expect_tx(bar, STAGE_BYTES);
         for (uint32_t pi = 0; pi < CK / PAGE; pi++) {
             // Pages past the sequence's last hold nothing this block may see (masked below): any valid page will do.
@@ -105,7 +115,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
         }
     };
     if (tid == 0)
-        for (uint32_t b = 0; b < min(n_blocks, STAGES); b++) issue(b);
+        for (uint32_t i = 0; i < min(my_blocks, STAGES); i++) issue(i);
 
     // Q fragments (A operands) straight from global memory: row g / g + 8, dims 16 ks + 2 tq (+ 8).
     uint32_t qa[4][4];
@@ -132,11 +142,11 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
         for (int e = 0; e < 4; e++) oacc[jd][e] = 0.0f;
 
     bool failed = false;
-    for (uint32_t b = 0; b < n_blocks; b++) {
-        const uint32_t st = b % STAGES, parity = (b / STAGES) & 1;
+    for (uint32_t i = 0; i < my_blocks; i++) {
+        const uint32_t b = i * GROUPS + grp, st = i % STAGES, parity = (i / STAGES) & 1;
         if (!mbar_wait(smem_u32(&bars[st]), parity)) { failed = true; }
-        if (__any_sync(0xffffffffu, failed)) { if (lane == 0) fail = 1; }
-        const uint32_t kbase = smem_u32(smem + st * STAGE_BYTES), vbase = kbase + CK * HD * 2, key0 = b * CK;
+        if (__any_sync(0xffffffffu, failed)) { if (lane == 0) fail[grp] = 1; }
+        const uint32_t kbase = smem_u32(ring + st * STAGE_BYTES), vbase = kbase + CK * HD * 2, key0 = b * CK;
         if (!failed && key0 < warp_end) {  // (a warp whose rows see nothing of this block skips the arithmetic, not the barriers)
             // S = Q K^T: 16 rows x 64 keys; n-tile j = keys 8 j .. 8 j + 7.
             float sacc[8][4];
@@ -210,17 +220,52 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
                 }
             }
         }
-        __syncthreads();  // every warp is done with this stage
-        if (fail) break;
-        if (tid == 0 && b + STAGES < n_blocks) issue(b + STAGES);
+        group_sync(grp);  // every warp of the group is done with this stage
+        if (fail[grp]) break;
+        if (tid == 0 && i + STAGES < my_blocks) issue(i + STAGES);
     }
-    if (fail) {
+    // The other groups' (m, l, O) to the first through their own rings (their copies have all been read), a float of every
+    // thread side by side; the first group adds them up in order and stores.
+    constexpr uint32_t ROW = WARPS * 32;
+    static_assert(36 * ROW * 4 <= STAGES * STAGE_BYTES, "a group's results must fit in its ring");
+    if (grp && !fail[grp]) {
+        float* mine = reinterpret_cast<float*>(ring) + tid;
+#pragma unroll
+        for (int jd = 0; jd < 8; jd++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) mine[(4 * jd + e) * ROW] = oacc[jd][e];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            mine[(32 + r) * ROW] = m_run[r];
+            mine[(34 + r) * ROW] = l_run[r];
+        }
+    }
+    __syncthreads();
+    bool any_fail = false;
+    for (uint32_t k = 0; k < GROUPS; k++) any_fail = any_fail || fail[k];
+    if (any_fail) {
         // A copy never arrived: say so, give the copies in flight a bounded time, and leave.
-        if (tid == 0) {
+        if (tid == 0 && fail[grp]) {
             atomicExch(a.err_flag, 3u);
             for (uint32_t s = 0; s < STAGES; s++) mbar_wait(smem_u32(&bars[s]), 0, 1u << 16);
         }
         return;
+    }
+    if (grp) return;
+#pragma unroll
+    for (uint32_t k = 1; k < GROUPS; k++) {
+        const float* theirs = reinterpret_cast<const float*>(smem + k * STAGES * STAGE_BYTES) + tid;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float m_other = theirs[(32 + r) * ROW], m_new = fmaxf(m_run[r], m_other), m_use = m_new == -INFINITY ? 0.0f : m_new;
+            const float w0 = fast_exp2(m_run[r] - m_use), w1 = fast_exp2(m_other - m_use);
+            m_run[r] = m_new;
+            l_run[r] = l_run[r] * w0 + theirs[(34 + r) * ROW] * w1;
+#pragma unroll
+            for (int jd = 0; jd < 8; jd++)
+#pragma unroll
+                for (int e = 2 * r; e < 2 * r + 2; e++) oacc[jd][e] = oacc[jd][e] * w0 + theirs[(4 * jd + e) * ROW] * w1;
+        }
     }
 #pragma unroll
     for (int r = 0; r < 2; r++) {
@@ -243,10 +288,10 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(ChunkAttnArgs a,
 
 void launch_attn_chunk(const ChunkAttnArgs& a, cudaStream_t s) {
     if (!a.n_ctiles) return;
-    const size_t smem = size_t(prefill::STAGES) * prefill::STAGE_BYTES + 1024;
+    const size_t smem = size_t(prefill::GROUPS) * prefill::STAGES * prefill::STAGE_BYTES + 1024;
     static PerDevice configured;
     configured.once([smem] { VLT_CUDA(cudaFuncSetAttribute(prefill::attn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); });
-    launch_pdl(prefill::attn_chunk_kernel, dim3(a.n_ctiles, a.n_heads), prefill::WARPS * 32, smem, s, a, *a.maps);
+    launch_pdl(prefill::attn_chunk_kernel, dim3(a.n_ctiles, a.n_heads), prefill::GROUPS * prefill::WARPS * 32, smem, s, a, *a.maps);
 }
 
 }  // namespace vlt

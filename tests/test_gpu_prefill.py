@@ -91,3 +91,28 @@ def test_a_computed_context_at_the_1b_dimensions_matches_the_oracle(tmp_path):
     errs.append(_agree_at_scale(prod, orc, [(a, rng.integers(0, vocab, 5).astype(np.uint32), E.Rows.ALL, False)], TOL[0]))
     print("1B dims, computed 8192-token context: logits error per step", [f"{e[0]:.2e}" for e in errs])
     prod.close()
+
+
+# Edges of a 64-key block and of the pair of key groups that share a chunk tile's blocks (9 .. 193 rows: one to four blocks,
+# odd counts leave the second group one less, a single block leaves it none), and of the GEMM's token blocks (two of 129 to
+# 256 tokens from 257 on, three from 513, four at 800; the last one short by up to its padding).
+@pytest.mark.parametrize("rows", [9, 64, 65, 128, 129, 193, 257, 272, 289, 511, 512, 513, 800])
+def test_a_chunk_at_the_edges_of_key_and_token_blocks_matches_the_oracle(rows):
+    w = util.weights("micro4", 0)
+    kw = dict(max_seqs=1, max_step_tokens=rows + 37, max_chunk=rows + 37, max_seq_len=2 * rows + 64, max_head_rows=rows + 37)
+    prod = E.Engine(w, E.EngineConfig(global_kv_tokens=2 * rows + 64, **kw))
+    orc = oracle.Engine(w, kv_tokens=2 * rows + 64, **kw)
+    a = prod.new_seq()
+    assert orc.new_seq() == a
+    rng = np.random.default_rng(rows)
+    vocab = prod.desc.vocab
+    prompt = rng.integers(0, vocab, 2 * rows).astype(np.uint32)
+    for chunk in (prompt[:rows], prompt[rows:]):  # the second one over cached keys, too
+        runs = [(a, chunk, E.Rows.ALL, False)]
+        out = prod.debug_step(runs, E.StepOptions(read_logits=True))
+        orc.step(runs)
+        want = orc.array("logits").reshape(-1, vocab)
+        assert float(np.abs(out.logits - want).max()) <= TOL[0]
+        same_state(prod, orc, 1, rows)
+    _caches_agree(prod, orc)
+    prod.close()
