@@ -542,31 +542,9 @@ void Engine::matmul_gemm(const Matrix& w, uint32_t n, const uint16_t* xb, float*
     a.ssq_in = ssq_in;
     a.ssq_tiles = ssq_in ? w.k / 128 : 0;
     a.ssq_stride = (cfg.max_step_tokens + 15) / 16 * 16;
-    // The kernel's N is at most 256 tokens: a longer step (a prompt chunk) goes in blocks of 256, the weights read once per
-    // block (the reference's tiled GEMM loops its token tiles the same way, kernels.metal:319-514). Everything indexed by
-    // token moves along with the block.
     if (side) a.side = *side;
-    const uint32_t out_w = epi == EPI_SIDE ? side->wide : epi_pairs(epi) ? w.m / 2 : w.m;
-    for (uint32_t t0 = 0; t0 < n; t0 += 256) {
-        MatArgs b = a;
-        b.n = std::min(256u, n - t0);
-        if (side) b.side.tokens = side->tokens + t0;
-        b.Xb = xb + size_t(t0) * w.k;
-        b.Y = y ? y + size_t(t0) * out_w : nullptr;
-        b.Yb = yb ? yb + size_t(t0) * out_w : nullptr;
-        b.base = base ? base + size_t(t0) * out_w : nullptr;
-        b.inv_in = inv ? inv + t0 : nullptr;
-        b.ssq_out = ssq_out ? ssq_out + t0 : nullptr;
-        b.ssq_in = ssq_in ? ssq_in + t0 : nullptr;
-        if (q) {
-            b.q.meta = q->meta + 2 * size_t(t0);
-            b.q.tin = q->tin + 2 * size_t(t0);
-            b.q.cpos = q->cpos ? q->cpos + t0 : nullptr;
-            b.q.q_b = q->q_b + size_t(t0) * q->n_heads * model.md.hd;
-        }
-        if (!gemm_supported(b)) throw Error("internal: GEMM asked for an unsupported shape");
-        launch_gemm(b, sm_count, s.err_flag.as<uint32_t>(), stream, !tuning.gemm_unpaired);
-    }
+    if (!gemm_supported(a)) throw Error("internal: GEMM asked for an unsupported shape");
+    launch_gemm(a, sm_count, s.err_flag.as<uint32_t>(), stream, !tuning.gemm_unpaired);
 }
 
 // engine/src/engine/encode.rs:142-192 `encode_layer`, a plain decoder's.

@@ -58,6 +58,8 @@ struct Args {
     uint32_t tmem_cols; // power of two >= 32 holding the accumulator and, for int8, the A stages
     uint32_t tmem_a0;   // int8: the first A stage's column (32 columns per stage)
     uint32_t splits;    // blocks of a cluster that share a weight tile, each over a slice of k
+    uint32_t t_first;   // this launch's first token ...
+    uint32_t t_blocks;  // ... and its blocks of n_pad tokens: every weight tile runs once per block
     uint32_t* err_flag;
 };
 
@@ -93,7 +95,8 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
     return v;
 }
 
-// grid: (m / 128) * splits blocks in clusters of `splits`. A cluster owns a 128-row weight tile;
+// grid: (m / 128) * t_blocks * splits blocks in clusters of `splits`. A cluster owns a 128-row weight tile for one block of
+// n_pad tokens (a tile's token blocks are neighbours in the grid: its weights come from HBM once);
 // its blocks each stream a slice of k into their own TMEM accumulator, send every group of 16 tokens
 // to the block that finishes it (stores into its shared memory), and each then adds up, in rank
 // order, the groups it owns.
@@ -128,7 +131,9 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
     auto stage_raw = [&](uint32_t r) { return smem_base + a_region + CB * b_bytes + r * raw_bytes; };
 
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const uint32_t rank = splits > 1 ? cluster_rank() : 0, tile = blockIdx.x / splits;
+    const uint32_t rank = splits > 1 ? cluster_rank() : 0, tile = blockIdx.x / splits / a.t_blocks;
+    // Token indices below are the block's own (shared memory, the accumulator's columns); t_base + t is the step's.
+    const uint32_t t_base = a.t_first + (blockIdx.x / splits % a.t_blocks) * n_pad, n_here = min(a.m.n - t_base, n_pad);
     const uint32_t row0 = tile * BM, nkb_all = a.m.k / BK;
     // This block's k blocks: an even share, the first ranks one more.
     const uint32_t kb_begin = rank * (nkb_all / splits) + min(rank, nkb_all % splits);
@@ -195,7 +200,7 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
                 if (!ok) break;
                 PROBE(3, i);
                 mbar_expect_tx(bar_bfull + 8 * c, b_bytes);
-                tma_load_2d(stage_b(c), &maps.b, int((kb_begin + i) * BK), 0, bar_bfull + 8 * c);
+                tma_load_2d(stage_b(c), &maps.b, int((kb_begin + i) * BK), int(t_base), bar_bfull + 8 * c);
                 if (++c == CB) { c = 0; ph ^= 1; }
             }
         }
@@ -329,9 +334,9 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
                 }
                 const uint32_t bits = f32_to_bf16(y), pair = bits | (__shfl_xor_sync(0xffffffffu, bits, 1) << 16);
                 const uint32_t t = t0 + j;
-                if (!valid || odd || t >= m.n) continue;  // the even lane writes the pair
+                if (!valid || odd || t >= n_here) continue;  // the even lane writes the pair
                 if (kind == 0) {
-                    *reinterpret_cast<uint32_t*>(qe.q_b + (size_t(t) * qe.n_heads + head) * 64 + d) = pair;
+                    *reinterpret_cast<uint32_t*>(qe.q_b + (size_t(t_base + t) * qe.n_heads + head) * 64 + d) = pair;
                 } else if (kvrow_s[t] != NO_TOK) {
                     const uint32_t g = kind == 1 ? head - qe.n_heads : head - qe.n_heads - qe.kv.n_kv;
                     uint16_t* cache = kind == 1 ? qe.k_cache : qe.v_cache;
@@ -345,7 +350,7 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
 #pragma unroll
         for (uint32_t j = 0; j < NTOK; j++) {
             inv[j] = inv_s[t0 + j];
-            base[j] = (EPI == EPI_RESID && m.base && valid && t0 + j < m.n) ? m.base[size_t(t0 + j) * m.m + row] : 0.0f;  // (no base: the sum alone, for its bf16 copy and sums of squares)
+            base[j] = (EPI == EPI_RESID && m.base && valid && t0 + j < n_here) ? m.base[size_t(t_base + t0 + j) * m.m + row] : 0.0f;  // (no base: the sum alone, for its bf16 copy and sums of squares)
         }
 #pragma unroll
         for (uint32_t j = 0; j < NTOK; j++) {
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
             else if (EPI == EPI_HEAD) y[j] = row < m.vocab_real ? x * inv[j] : -INFINITY;
             else if (EPI == EPI_HEAD_CAP) y[j] = row < m.vocab_real ? 23.0f * (1.0f / (1.0f + __expf(-(x + 5.0f) / 7.5f))) : -INFINITY;  // kernels.metal:196-199
             else if (EPI == EPI_RELU2) y[j] = x > 0.0f ? x * x : 0.0f;
-            else if (EPI == EPI_SIDE) y[j] = t0 + j < m.n ? side_of(m.side, t0 + j, row, x) : 0.0f;
+            else if (EPI == EPI_SIDE) y[j] = t0 + j < n_here ? side_of(m.side, t_base + t0 + j, row, x) : 0.0f;
             else if (EPI == EPI_SILU) y[j] = row < m.vocab_real ? x * __fdividef(1.0f, 1.0f + __expf(-x)) : x;
             else y[j] = x;
         }
@@ -391,8 +396,8 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
         if (writes) {
 #pragma unroll
             for (uint32_t j = 0; j < NTOK; j++)
-                if (t0 + j < m.n) {
-                    const size_t o = size_t(t0 + j) * out_w + out_r;
+                if (t0 + j < n_here) {
+                    const size_t o = size_t(t_base + t0 + j) * out_w + out_r;
                     if (m.Y) m.Y[o] = y[j];
                     if (m.Yb) m.Yb[o] = f32_to_bf16(y[j]);
                 }
@@ -403,36 +408,35 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
     auto write_ssq = [&](uint32_t t_lo, uint32_t t_hi) {
         asm volatile("bar.sync 1, %0;" ::"n"(32 * CONV_WARPS) : "memory");  // every epilogue warp, whatever happened before: the row groups' sums are in
         if (*abort_flag) return;
-        for (uint32_t t = t_lo + tid - FIRST_CONV * 32; t < t_hi && t < m.n; t += 32 * CONV_WARPS)
-            m.ssq_out[size_t(tile) * m.ssq_stride + t] = ((ssq_s[t] + ssq_s[n_pad + t]) + ssq_s[2 * n_pad + t]) + ssq_s[3 * n_pad + t];
+        for (uint32_t t = t_lo + tid - FIRST_CONV * 32; t < t_hi && t < n_here; t += 32 * CONV_WARPS)
+            m.ssq_out[size_t(tile) * m.ssq_stride + t_base + t] = ((ssq_s[t] + ssq_s[n_pad + t]) + ssq_s[2 * n_pad + t]) + ssq_s[3 * n_pad + t];
     };
 
     if (warp >= FIRST_CONV) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         for (uint32_t t = tid - FIRST_CONV * 32; t < n_pad; t += 32 * CONV_WARPS) {
             float inv = 1.0f;
-            if (t < a.m.n) {
-                if (a.m.inv_in) inv = a.m.inv_in[t];
+            if (t < n_here) {
+                if (a.m.inv_in) inv = a.m.inv_in[t_base + t];
                 else if (a.m.ssq_in) {  // the tiles' sums in tile order
                     float ss = 0.0f;
-                    for (uint32_t tl = 0; tl < a.m.ssq_tiles; tl++) ss += a.m.ssq_in[size_t(tl) * a.m.ssq_stride + t];
+                    for (uint32_t tl = 0; tl < a.m.ssq_tiles; tl++) ss += a.m.ssq_in[size_t(tl) * a.m.ssq_stride + t_base + t];
                     inv = rsqrtf(ss / float(a.m.k) + a.m.eps);
                 }
             }
             inv_s[t] = inv;
-            if (EPI == EPI_SIDE && t < a.m.n && row0 < a.m.side.dim) {  // the table's entries for this tile on their way while the products run
-                const uint16_t* e = a.m.side.table + size_t(a.m.side.tokens[t]) * a.m.side.ld + a.m.side.first + row0;
+            if (EPI == EPI_SIDE && t < n_here && row0 < a.m.side.dim) {  // the table's entries for this tile on their way while the products run
+                const uint16_t* e = a.m.side.table + size_t(a.m.side.tokens[t_base + t]) * a.m.side.ld + a.m.side.first + row0;
                 for (uint32_t i = 0; i < min(BM, a.m.side.dim - row0); i += 64) asm volatile("prefetch.global.L1 [%0];" ::"l"(e + i));
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(e + min(BM, a.m.side.dim - row0) - 1));
             }
             if (EPI == EPI_QKV) {
                 const QkvEpilogue& qe = a.m.q;
                 uint32_t pos = 0, kvrow = NO_TOK;
-                if (t < a.m.n) {
-                    const uint32_t slot = qe.meta[2 * t], row = qe.tin[2 * t + 1];
-                    pos = qe.meta[2 * t + 1];
-                    // (the run's first token may lie before this launch's block of tokens: a signed index)
-                    const uint32_t cp = qe.cpos ? qe.cpos[t] : qe.meta[2 * (int(t) - int(row)) + 1] + row;  // kernels.metal:74-77 `cache_pos`
+                if (t < n_here) {
+                    const uint32_t st = t_base + t, slot = qe.meta[2 * st], row = qe.tin[2 * st + 1];
+                    pos = qe.meta[2 * st + 1];
+                    const uint32_t cp = qe.cpos ? qe.cpos[st] : qe.meta[2 * (st - row) + 1] + row;  // kernels.metal:74-77 `cache_pos`
                     if (cp != NO_TOK) {
                         const uint32_t page = qe.page_table[size_t(slot) * qe.kv.max_pages + (cp >> qe.kv.page_shift)], psize = 1u << qe.kv.page_shift;
                         kvrow = ((qe.layer * qe.kv.n_pages + page) * qe.kv.n_kv) * psize + (cp & (psize - 1));
@@ -528,9 +532,9 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
 
 }  // namespace gemm
 
-// Tensor maps are made once per (operand pointer, shape) and kept: the engine's buffers never move.
+// Tensor maps are made once per (operand pointers, shape, tokens, tokens a block) and kept: the engine's buffers never move.
 struct GemmMapCache {
-    std::map<std::tuple<const void*, const void*, uint32_t, uint32_t, uint32_t>, gemm::Maps> maps;
+    std::map<std::tuple<const void*, const void*, uint32_t, uint32_t, uint32_t, uint32_t>, gemm::Maps> maps;
 };
 
 typedef void (*GemmEntry)(const gemm::Maps, const gemm::Args);
@@ -554,22 +558,52 @@ static GemmEntry gemm_entry(bool int8, uint32_t epi, bool paired = false) {
 
 bool gemm_supported(const MatArgs& a) {
     const bool grouped = a.int8 && a.group < a.k;  // scale groups: powers of two from 8
-    return a.n >= 1 && a.n <= 256 && a.m % gemm::BM == 0 && a.k % gemm::BK == 0 && (!grouped || (a.group >= 8 && !(a.group & (a.group - 1)))) && a.Xb != nullptr &&
+    return a.n >= 1 && a.m % gemm::BM == 0 && a.k % gemm::BK == 0 && (!grouped || (a.group >= 8 && !(a.group & (a.group - 1)))) && a.Xb != nullptr &&
            (a.epi == EPI_RESID || a.epi == EPI_RAW || a.epi == EPI_HEAD_CAP || a.epi == EPI_RELU2 ||
             (!a.int8 && (a.epi == EPI_SILU || a.epi == EPI_GLU || a.epi == EPI_GLU_CLAMP || a.epi == EPI_SIDE)) || a.inv_in != nullptr || a.ssq_in != nullptr);
+}
+
+// Split k over a cluster when the tiles alone cannot fill the SMs (the reference splits K the same way when a GEMM has few
+// tiles, encode.rs:545-553): the most blocks a tile can have with every cluster resident at once. 1 where there are more
+// tiles than SMs.
+static uint32_t k_splits(const MatArgs& a, uint32_t tiles, uint32_t nkb, uint32_t sm_count, size_t smem) {
+    static thread_local std::map<std::tuple<bool, uint32_t, uint32_t>, uint32_t> wave;  // (int8, smem, cluster size) -> clusters one wave holds
+    uint32_t splits = std::max(1u, std::min(8u, std::min(sm_count / tiles, nkb)));
+    for (; splits > 1; splits--) {
+        auto wk = std::make_tuple(a.int8, uint32_t(smem) * 16 + a.epi, splits);
+        auto w = wave.find(wk);
+        if (w == wave.end()) {
+            cudaLaunchConfig_t q = {};
+            q.gridDim = dim3(tiles * splits);
+            q.blockDim = dim3(gemm::threads_of(16));
+            q.dynamicSmemBytes = smem;
+            cudaLaunchAttribute qa[1];
+            qa[0].id = cudaLaunchAttributeClusterDimension;
+            qa[0].val.clusterDim.x = splits;
+            qa[0].val.clusterDim.y = qa[0].val.clusterDim.z = 1;
+            q.attrs = qa;
+            q.numAttrs = 1;
+            int n_clusters = 0;
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n_clusters, gemm_entry(a.int8, a.epi), &q);
+            w = wave.emplace(wk, e == cudaSuccess ? uint32_t(n_clusters) : 0u).first;
+        }
+        if (tiles <= w->second) break;  // every cluster is resident at once
+    }
+    return splits;
 }
 
 void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired) {
     static thread_local GemmMapCache cache;
     static PerDevice configured;
-    const uint32_t n_pad = (a.n + 15) / 16 * 16;
-    auto key = std::make_tuple(static_cast<const void*>(a.W), static_cast<const void*>(a.Xb), a.m, a.k, n_pad);
+    // The MMA's N is at most 256 tokens: a longer step goes in equal blocks of at most that many.
+    const uint32_t n_blocks = (a.n + 255) / 256, n_pad = ((a.n + n_blocks - 1) / n_blocks + 15) / 16 * 16, n_rows = (a.n + 15) / 16 * 16;
+    auto key = std::make_tuple(static_cast<const void*>(a.W), static_cast<const void*>(a.Xb), a.m, a.k, n_rows, n_pad);
     auto it = cache.maps.find(key);
     if (it == cache.maps.end()) {
         gemm::Maps m;
         if (a.int8) make_tensor_map_2d(m.a, a.W, a.k, a.m, gemm::BK, gemm::BM, 1, false, true);
         else make_tensor_map_2d(m.a, a.W, a.k, a.m, gemm::BK, gemm::BM, 2, true);
-        make_tensor_map_2d(m.b, a.Xb, a.k, n_pad, gemm::BK, n_pad, 2, true);
+        make_tensor_map_2d(m.b, a.Xb, a.k, n_rows, gemm::BK, n_pad, 2, true);  // (a last block's rows past the end read as zeros)
         it = cache.maps.emplace(key, m).first;
     }
     // Shared memory: B stages of n_pad x 128 B; bf16 weights, as many A stages of 16 KiB; int8 weights, A
@@ -603,29 +637,16 @@ void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaSt
         VLT_CUDA(cudaFuncSetAttribute(gemm_entry(true, EPI_HEAD, true), cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
         VLT_CUDA(cudaFuncSetAttribute(gemm_entry(true, EPI_HEAD, true), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     });
-    // Split k over a cluster when the tiles alone cannot fill the SMs (the reference splits K the
-    // same way when a GEMM has few tiles, encode.rs:545-553).
-    static thread_local std::map<std::tuple<bool, uint32_t, uint32_t>, uint32_t> wave;  // (int8, smem, cluster size) -> clusters one wave holds
-    uint32_t splits = std::max(1u, std::min(8u, std::min(sm_count / tiles, nkb)));  // (1 for a paired launch: more tiles than SMs)
-    for (; splits > 1; splits--) {
-        auto wk = std::make_tuple(a.int8, uint32_t(smem) * 16 + a.epi, splits);
-        auto w = wave.find(wk);
-        if (w == wave.end()) {
-            cudaLaunchConfig_t q = {};
-            q.gridDim = dim3(tiles * splits);
-            q.blockDim = dim3(gemm::threads_of(16));
-            q.dynamicSmemBytes = smem;
-            cudaLaunchAttribute qa[1];
-            qa[0].id = cudaLaunchAttributeClusterDimension;
-            qa[0].val.clusterDim.x = splits;
-            qa[0].val.clusterDim.y = qa[0].val.clusterDim.z = 1;
-            q.attrs = qa;
-            q.numAttrs = 1;
-            int n_clusters = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n_clusters, gemm_entry(a.int8, a.epi), &q);
-            w = wave.emplace(wk, e == cudaSuccess ? uint32_t(n_clusters) : 0u).first;
-        }
-        if (tiles <= w->second) break;  // every cluster is resident at once
+    // How many token blocks a launch takes. Together they share its fixed part (fill, the split-k exchange, epilogue, the
+    // gap to the next launch: about as long as FIXED k blocks) and exchange fewer partial sums, since more blocks means
+    // fewer splits; apart, a matrix whose tiles fill the SMs badly keeps more of them busy. The cheaper by this count.
+    constexpr double FIXED = 20.0;
+    uint32_t together = n_blocks;
+    double best = 1e30;
+    for (uint32_t g = n_blocks; g >= 1; g--) {
+        const uint32_t sp = k_splits(a, tiles * g, nkb, sm_count, smem), waves = (tiles * g * sp + sm_count - 1) / sm_count;
+        const double cost = double((n_blocks + g - 1) / g) * (double(waves) * ((nkb + sp - 1) / sp) + FIXED);
+        if (cost < best) { best = cost; together = g; }
     }
     gemm::Args g;
     g.m = a;
@@ -637,34 +658,38 @@ void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaSt
     while (cols < (a.int8 ? tmem_a0 + 32 * stages_a : n_pad)) cols *= 2;
     g.tmem_cols = cols;
     g.tmem_a0 = tmem_a0;
-    g.splits = splits;
     g.err_flag = err_flag;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles * splits);
-    cfg.blockDim = dim3(gemm::threads_of(paired ? 8 : 16));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // may start while the kernel before it drains
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = splits;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = splits > 1 ? 2 : 1;
-    VLT_CUDA(cudaLaunchKernelEx(&cfg, gemm_entry(a.int8, a.epi, paired), it->second, g));
-    launch_counter()++;
+    for (uint32_t b0 = 0; b0 < n_blocks; b0 += together) {
+        g.t_first = b0 * n_pad;
+        g.t_blocks = std::min(together, n_blocks - b0);
+        const uint32_t splits = g.splits = k_splits(a, tiles * g.t_blocks, nkb, sm_count, smem);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(tiles * g.t_blocks * splits);
+        cfg.blockDim = dim3(gemm::threads_of(paired ? 8 : 16));
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // may start while the kernel before it drains
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = splits;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = splits > 1 ? 2 : 1;
+        VLT_CUDA(cudaLaunchKernelEx(&cfg, gemm_entry(a.int8, a.epi, paired), it->second, g));
+        launch_counter()++;
+    }
 #ifdef VLT_GEMM_PROBE
     if (getenv("VLT_GEMM_PROBE")) {
         cudaStreamSynchronize(s);
         static unsigned long long h[8][64];
         cudaMemcpyFromSymbol(h, gemm::g_probe, sizeof(h));
-        fprintf(stderr, "gemm m=%u k=%u n=%u splits=%u stages a %u b %u raw %u\n", a.m, a.k, a.n, splits, stages_a, stages_b, raw_stages);
+        fprintf(stderr, "gemm m=%u k=%u n=%u splits=%u stages a %u b %u raw %u\n", a.m, a.k, a.n, g.splits, stages_a, stages_b, raw_stages);
         const unsigned long long t0 = h[0][0];
         fprintf(stderr, "epilogue (ns from the first weight load): starts %lld accumulator done %lld dumped %lld cluster barrier %lld summed %lld emitted %lld left %lld\n",
                 (long long)(h[7][0] - t0), (long long)(h[7][1] - t0), (long long)(h[7][2] - t0), (long long)(h[7][3] - t0), (long long)(h[7][4] - t0), (long long)(h[7][5] - t0), (long long)(h[7][6] - t0));
-        for (uint32_t i = 0; i < std::min(64u, nkb / splits); i++)
+        for (uint32_t i = 0; i < std::min(64u, nkb / g.splits); i++)
             fprintf(stderr, "kb %2u: tmaA %6lld convstart %6lld convdone %6lld tmaB %6lld afull %6lld bfull %6lld commit %6lld\n", i, (long long)(h[0][i] - t0),
                     (long long)(h[1][i] - t0), (long long)(h[2][i] - t0), (long long)(h[3][i] - t0), (long long)(h[4][i] - t0), (long long)(h[5][i] - t0), (long long)(h[6][i] - t0));
     }
