@@ -236,9 +236,16 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    // The items in order are (row tile, slice) pairs; every walk over them counts on instead of dividing: the loop below is
+    // bound by instruction issue, and four divisions an item in each of 16 warps are some 100 instructions of 400.
+    auto next = [&](uint32_t& rt, uint32_t& sl) {
+        if (++sl == slices) {
+            sl = 0;
+            rt += gridDim.x;
+        }
+    };
     // One warp requests an item: lane 0 announces the bytes, lanes 0..15 copy a row piece each.
-    auto request = [&](uint32_t item) {
-        const uint32_t rt = blockIdx.x + (item / slices) * gridDim.x, sl = item % slices, st = item % n_stages;
+    auto request = [&](uint32_t rt, uint32_t sl, uint32_t st) {
         const uint32_t bytes = (min(n_tiles - sl * 32, 32u)) * 64, bar = st_smem_u32(&bars[st]);
         if (lane == 0) st_mbar_expect_tx(bar, bytes * 16);
         __syncwarp();
@@ -249,8 +256,7 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
     if (tid == 0) SP_TIME(sp_t[0]);
     // Another warp asks L2 for an item some items before it is asked for into a stage: a block that is resident early
     // (while the kernel before still runs) then has HBM work on more than its stages hold.
-    auto prefetch = [&](uint32_t item) {
-        const uint32_t rt = blockIdx.x + (item / slices) * gridDim.x, sl = item % slices;
+    auto prefetch = [&](uint32_t rt, uint32_t sl) {
         const uint32_t bytes = (min(n_tiles - sl * 32, 32u)) * 64;
         if (lane < 16) {
             const uint8_t* src = a.W + size_t(rt * 16 + lane) * row_bytes + size_t(sl) * STREAM_SLICE;
@@ -259,10 +265,17 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
     };
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // (The requesting warps are not among the four that add up and store a row tile: asking takes a while.)
-    if (warp == NW - 1)
-        for (uint32_t i = 0; i < min(n_stages, n_items); i++) request(i);
+    uint32_t q_rt = blockIdx.x, q_sl = 0;  // the next item that this warp, if it is one of the two, asks for
+    if (warp >= NW - 2)
+        for (uint32_t i = 0; i < min(n_stages, n_items); i++) {
+            if (warp == NW - 1) request(q_rt, q_sl, i);
+            next(q_rt, q_sl);
+        }
     if (warp == NW - 2)
-        for (uint32_t i = n_stages; i < min(n_stages + STREAM_AHEAD, n_items); i++) prefetch(i);
+        for (uint32_t i = n_stages; i < min(n_stages + STREAM_AHEAD, n_items); i++) {
+            prefetch(q_rt, q_sl);
+            next(q_rt, q_sl);
+        }
     // The rows' scales are read once each, so every row tile would wait for HBM in its turn: all of them now.
     if (INT8 && !grouped)
         for (uint32_t i = tid; i < min(my_row_tiles, STREAM_SCALE_TILES) * 16; i += 512)
@@ -393,12 +406,13 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     uint32_t buf = 0;
     const bool has_x = g < a.n;
+    uint32_t rt = blockIdx.x, sl = 0, st = 0, ph = 0, done_tiles = 0;  // the item's row tile and slice, its stage and that stage's phase, row tiles behind it
     for (uint32_t item = 0; item < n_items; item++) {
-        const uint32_t rt = blockIdx.x + (item / slices) * gridDim.x, sl = item % slices, st = item % n_stages, row0 = rt * 16;
+        const uint32_t row0 = rt * 16;
         const uint32_t count = min(n_tiles - sl * 32, 32u);  // 64-byte tiles in this slice
         // One scale per row, applied once after the sum (from shared memory; past its room, asked for before the wait).
         float row_sl = 1.0f, row_sh = 1.0f;
-        if (INT8 && !grouped && sl + 1 == slices && item / slices >= STREAM_SCALE_TILES) {
+        if (INT8 && !grouped && sl + 1 == slices && done_tiles >= STREAM_SCALE_TILES) {
             row_sl = bf16_to_f32(a.scales[row0 + g]);
             row_sh = bf16_to_f32(a.scales[row0 + g + 8]);
         }
@@ -406,7 +420,7 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
         float resid = 0.0f, bias = 0.0f;
         if (!INT8 && a.bias && sl + 1 == slices && tid < 128) bias = bf16_to_f32(a.bias[row0 + tid % 16]);
         if (a.epi == EPI_RESID && sl + 1 == slices && tid < 128 && tid / 16 < a.n) resid = a.base[size_t(tid / 16) * a.m + row0 + tid % 16];
-        if (!st_mbar_wait(st_smem_u32(&bars[st]), (item / n_stages) & 1) && lane == 0 && a.err_flag) atomicExch(a.err_flag, 2u);
+        if (!st_mbar_wait(st_smem_u32(&bars[st]), ph) && lane == 0 && a.err_flag) atomicExch(a.err_flag, 2u);
         const uint8_t* sw = stages + size_t(st) * STREAM_STAGE;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -452,9 +466,9 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
             }
         }
         if (sl + 1 == slices) {  // the row tile is complete: add up the warps and store
-            if (INT8 && !grouped && item / slices < STREAM_SCALE_TILES) {
-                row_sl = row_scale[(item / slices) * 16 + g];
-                row_sh = row_scale[(item / slices) * 16 + g + 8];
+            if (INT8 && !grouped && done_tiles < STREAM_SCALE_TILES) {
+                row_sl = row_scale[done_tiles * 16 + g];
+                row_sh = row_scale[done_tiles * 16 + g + 8];
             }
             acc[0] *= row_sl; acc[1] *= row_sl; acc[2] *= row_sh; acc[3] *= row_sh;
             float* rb = red + size_t(buf) * NW * 128 + warp * 128;  // [row][token]
@@ -465,8 +479,14 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
             acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
         }
         __syncthreads();  // every warp is done with the stage (and, after a row tile, has left its sums)
-        if (warp == NW - 1 && item + n_stages < n_items) request(item + n_stages);
-        if (warp == NW - 2 && item + n_stages + STREAM_AHEAD < n_items) prefetch(item + n_stages + STREAM_AHEAD);
+        if (warp == NW - 1 && item + n_stages < n_items) {  // into the stage that just came free
+            request(q_rt, q_sl, st);
+            next(q_rt, q_sl);
+        }
+        if (warp == NW - 2 && item + n_stages + STREAM_AHEAD < n_items) {
+            prefetch(q_rt, q_sl);
+            next(q_rt, q_sl);
+        }
         if (sl + 1 == slices) {
             // Warps 0..3: thread (token b, row r), consecutive threads on consecutive rows of one token. The buffer
             // alternates: a warp can be one row tile ahead of the four that are still adding up, never two.
@@ -518,6 +538,12 @@ __global__ void __launch_bounds__(512, 2) matmul_stream_kernel(MatArgs a, uint32
                 }
             }
             buf ^= 1;
+            done_tiles++;
+        }
+        next(rt, sl);
+        if (++st == n_stages) {
+            st = 0;
+            ph ^= 1;
         }
     }
     if (tid == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1)) {
