@@ -1,5 +1,5 @@
 // The verify GEMM on the 5th-generation tensor cores: Y[t][row] = epilogue(W[row] . Xb[t]) for
-// steps of 16 to 256 tokens (S streams x k+1 rows). The reference's tiled GEMM
+// steps of 9 tokens or more (S streams x k+1 rows, portions of prompts). The reference's tiled GEMM
 // (kernels.metal:319-514) stages k tiles through threadgroup memory and dequantises on the way;
 // here
 //   - the weight tile is the MMA's M side (128 rows) and the tokens its N side (16..256), so a
