@@ -128,7 +128,8 @@ __device__ __forceinline__ float row_max(const RowWork& w) {
 // 32 groups of 32 threads; with a q row its draft id, read here once (an id past the vocabulary as 0, see
 // launch_spec_accept_static). The row is read from memory once. A thread stands for two neighbours of the 1024, whose sums
 // are the halves of packed registers; the maximum is taken on packed bf16, whoever's ids they are. What the cluster has to
-// agree on is the maximum alone: every block stores its own into the others and there is one barrier.
+// agree on is the maximum alone: every block stores its own into the others, which a first cluster barrier, under way while the
+// row comes in, knows to have started, and a second one says that the maxima are there.
 // What bounds it: a row's 256 KiB of shared memory let 131 rows run at a time, and such a wave takes 5 us of HBM, 5 us of the
 // fp32 pipe (11 packed operations for two ids) and a barrier one after another. Three kernels without clusters that read the
 // row twice (maxima; sums; decision) took 24 / 67 us with the decision at 18 / 288 rows of 128 256 ids, one block per row
@@ -139,6 +140,7 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(STATS_THREADS)
                                                                                            const uint32_t* __restrict__ drafts, uint32_t p_rows, uint32_t vocab, bool vec,
                                                                                            float c, RowWork* work) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // "this block is there": waited for before the first store to another one
     extern __shared__ __align__(16) uint16_t row_sm[];
     __shared__ float maxima[SC_CTAS];
     __shared__ uint32_t wbv[STATS_THREADS / 32], first_id;
@@ -174,6 +176,7 @@ __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(STATS_THREADS)
 #pragma unroll
     for (uint32_t w = 0; w < STATS_THREADS / 32; w++) best = max_bf16x2(best, wbv[w]);
     const float mine = fmaxf(-FLT_MAX, fmaxf(bf16lo(best), bf16hi(best)));
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // (long over, but for a short row: its later blocks have no id to load)
     if (tid < SC_CTAS) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sc_remote(&maxima[rank], tid)), "f"(mine) : "memory");
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     {  // meanwhile the lowest id of the share's own best
