@@ -544,7 +544,7 @@ void Engine::matmul_gemm(const Matrix& w, uint32_t n, const uint16_t* xb, float*
     a.ssq_stride = (cfg.max_step_tokens + 15) / 16 * 16;
     if (side) a.side = *side;
     if (!gemm_supported(a)) throw Error("internal: GEMM asked for an unsupported shape");
-    launch_gemm(a, sm_count, s.err_flag.as<uint32_t>(), stream, !tuning.gemm_unpaired);
+    launch_gemm(a, gemm_maps, sm_count, s.err_flag.as<uint32_t>(), stream, !tuning.gemm_unpaired);
 }
 
 // engine/src/engine/encode.rs:142-192 `encode_layer`, a plain decoder's.

@@ -223,6 +223,7 @@ class Engine {
     Buffer rope_tab;
     Buffer spec_p, spec_q, spec_small;  // spec_accept's device copies, grown on demand
     AttnMaps attn_maps;
+    GemmMaps gemm_maps;  // of this engine's buffers
     // The chain drafter (a benchmark extension; the reference's drafter.rs is a block drafter): fc over
     // (feature ; embedding), one decoder layer with a cache of its own on the target's page table, a head
     // over a draft vocabulary.

@@ -25,7 +25,7 @@ namespace vlt {
 
 namespace gemm {
 
-constexpr uint32_t BM = 128, BK = 64;
+constexpr uint32_t BM = GemmMaps::BM, BK = GemmMaps::BK;
 constexpr uint32_t CONV_WPG = 4;  // converter warps per group: one per quarter of the TMEM lanes
 constexpr uint32_t FIRST_CONV = 3;
 // warp 0: weight TMA, warp 1: MMA, warp 2: activation TMA, the rest (CW of them, in groups that each take their own k
@@ -44,10 +44,7 @@ __device__ __forceinline__ void cvt_i8x4(uint32_t w, uint32_t& lo, uint32_t& hi)
     hi = __byte_perm(__float_as_uint(f2), __float_as_uint(f3), 0x7632);
 }
 
-struct Maps {
-    alignas(64) uint8_t a[128];
-    alignas(64) uint8_t b[128];
-};
+typedef GemmMapPair Maps;
 
 struct Args {
     MatArgs m;
@@ -532,11 +529,6 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
 
 }  // namespace gemm
 
-// Tensor maps are made once per (operand pointers, shape, tokens, tokens a block) and kept: the engine's buffers never move.
-struct GemmMapCache {
-    std::map<std::tuple<const void*, const void*, uint32_t, uint32_t, uint32_t, uint32_t>, gemm::Maps> maps;
-};
-
 typedef void (*GemmEntry)(const gemm::Maps, const gemm::Args);
 static GemmEntry gemm_entry(bool int8, uint32_t epi, bool paired = false) {
     if (paired) return gemm::gemm_kernel<true, EPI_HEAD, 8>;  // the only shape that runs in waves
@@ -592,20 +584,11 @@ static uint32_t k_splits(const MatArgs& a, uint32_t tiles, uint32_t nkb, uint32_
     return splits;
 }
 
-void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired) {
-    static thread_local GemmMapCache cache;
+void launch_gemm(const MatArgs& a, GemmMaps& maps, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired) {
     static PerDevice configured;
     // The MMA's N is at most 256 tokens: a longer step goes in equal blocks of at most that many.
     const uint32_t n_blocks = (a.n + 255) / 256, n_pad = ((a.n + n_blocks - 1) / n_blocks + 15) / 16 * 16, n_rows = (a.n + 15) / 16 * 16;
-    auto key = std::make_tuple(static_cast<const void*>(a.W), static_cast<const void*>(a.Xb), a.m, a.k, n_rows, n_pad);
-    auto it = cache.maps.find(key);
-    if (it == cache.maps.end()) {
-        gemm::Maps m;
-        if (a.int8) make_tensor_map_2d(m.a, a.W, a.k, a.m, gemm::BK, gemm::BM, 1, false, true);
-        else make_tensor_map_2d(m.a, a.W, a.k, a.m, gemm::BK, gemm::BM, 2, true);
-        make_tensor_map_2d(m.b, a.Xb, a.k, n_rows, gemm::BK, n_pad, 2, true);  // (a last block's rows past the end read as zeros)
-        it = cache.maps.emplace(key, m).first;
-    }
+    const gemm::Maps& pair = maps.get(a.W, a.Xb, a.m, a.k, a.int8, n_rows, n_pad);
     // Shared memory: B stages of n_pad x 128 B; bf16 weights, as many A stages of 16 KiB; int8 weights, A
     // stages in tensor memory behind the accumulator and raw stages of 8 KiB in the shared memory left.
     const uint32_t a_bytes = gemm::BM * gemm::BK * 2, b_bytes = n_pad * gemm::BK * 2, raw_bytes = gemm::BM * gemm::BK;
@@ -677,7 +660,7 @@ void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaSt
         attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = splits > 1 ? 2 : 1;
-        VLT_CUDA(cudaLaunchKernelEx(&cfg, gemm_entry(a.int8, a.epi, paired), it->second, g));
+        VLT_CUDA(cudaLaunchKernelEx(&cfg, gemm_entry(a.int8, a.epi, paired), pair, g));
         launch_counter()++;
     }
 #ifdef VLT_GEMM_PROBE

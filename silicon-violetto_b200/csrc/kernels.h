@@ -5,6 +5,7 @@
 #include "common.h"
 #include "device.cuh"
 #include "layered.h"
+#include "tensor_maps.h"
 #include "weights.h"
 
 namespace vlt {
@@ -118,8 +119,6 @@ struct alignas(64) AttnMaps {
     alignas(64) uint8_t v[128];
 };
 void attn_maps_init(AttnMaps* m, const uint16_t* k_cache, const uint16_t* v_cache, uint64_t total_rows);
-void make_tensor_map_2d(void* out_map, const void* base, uint64_t inner, uint64_t rows, uint32_t box_inner, uint32_t box_rows, uint32_t elem_bytes,
-                        bool swizzle128, bool swizzle64 = false);
 struct AttnArgs {
     const AttnMaps* maps;  // host pointer
     uint32_t* err_flag;    // device word set if a bounded wait ran out
@@ -235,7 +234,7 @@ void launch_limite_compact(const RunIn* runs, const uint32_t* path, const uint32
 // The tcgen05 GEMM for 16..256 tokens: needs Xb (bf16 X, rows padded to 16), inv_in for the
 // normed epilogues, m a multiple of 128, one int8 scale per row.
 bool gemm_supported(const MatArgs& a);
-void launch_gemm(const MatArgs& a, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired = true);
+void launch_gemm(const MatArgs& a, GemmMaps& maps, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired = true);
 void launch_matmul_stream(const MatArgs& a, uint32_t sm_count, cudaStream_t s);  // n <= 8, tensor cores fed from registers
 bool matmul_stream_fits(const MatArgs& a);                                      // else launch_matmul_stream falls back to the scalar kernel
 void launch_matmul_rows(const MatArgs& a, cudaStream_t s);                      // any n, scalar (cross-check, odd scale groups)
