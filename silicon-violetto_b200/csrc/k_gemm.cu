@@ -622,11 +622,15 @@ void launch_gemm(const MatArgs& a, GemmMaps& maps, uint32_t sm_count, uint32_t* 
     });
     // How many token blocks a launch takes. Together they share its fixed part (fill, the split-k exchange, epilogue, the
     // gap to the next launch: about as long as FIXED k blocks) and exchange fewer partial sums, since more blocks means
-    // fewer splits; apart, a matrix whose tiles fill the SMs badly keeps more of them busy. The cheaper by this count.
-    constexpr double FIXED = 20.0;
+    // fewer splits; apart, a matrix whose tiles fill the SMs badly keeps more of them busy, which pays off where k is long.
+    // FIXED is where the two meet, from matrices of 20 to 40 row tiles timed both ways (int8, us; bf16 the same within 10 %):
+    // 40 tiles of k 5 120, 512 tokens: 36 together, 42 apart; 24 tiles of k 14 336, 512 tokens: 48 and 58; 28 tiles of
+    // k 14 336, 768 tokens: 84 and 94; 24 tiles of k 14 336, 2 048 tokens: 173 together, 148 in threes; 20 tiles of
+    // k 28 672, 1 024 tokens: 154 together, 123 in twos. The first three and the last put it between 48 and 75.
+    constexpr double FIXED = 50.0;
     uint32_t together = n_blocks;
     double best = 1e30;
-    for (uint32_t g = n_blocks; g >= 1; g--) {
+    for (uint32_t g = n_blocks; g >= 1 && n_blocks > 1; g--) {
         const uint32_t sp = k_splits(a, tiles * g, nkb, sm_count, smem), waves = (tiles * g * sp + sm_count - 1) / sm_count;
         const double cost = double((n_blocks + g - 1) / g) * (double(waves) * ((nkb + sp - 1) / sp) + FIXED);
         if (cost < best) { best = cost; together = g; }
