@@ -409,6 +409,7 @@ Plan Engine::plan(uint32_t set, const std::vector<PlanRun>& runs, Rows hidden) {
         for (uint32_t i = 0; i < count; i += 64) {
             ctiles.push_back(first_row + i);
             ctiles.push_back(std::min(count - i, 64u));
+            p.ckey_blocks += (sq.len + std::min(i + 64, count) + 63) / 64;
         }
         max_keys = std::max(max_keys, new_len);
         max_count = std::max(max_count, count);
@@ -561,6 +562,7 @@ void Engine::encode_layer(uint32_t set, const Plan& p, uint32_t li, bool capture
     io.n_tiles = p.tiles;
     io.ctiles = st.in<uint32_t>(st.o_ctiles);
     io.n_ctiles = p.chunked ? p.ctiles : 0;
+    io.ckey_blocks = p.ckey_blocks;
     io.k_cache = kv.k.as<uint16_t>();
     io.v_cache = kv.v.as<uint16_t>();
     io.maps = &attn_maps;
@@ -661,7 +663,7 @@ void Engine::encode_layer_io(const LayerIO& io, bool capture) {
         c.out = s.attn.as<float>();
         c.out_b = s.attn_b.as<uint16_t>();
         sp = span_begin(G_ATTN);
-        if (!(skip & 4)) launch_attn_chunk(c, stream);
+        if (!(skip & 4)) launch_attn_chunk(c, io.ckey_blocks, sm_count, stream);
         span_end(sp);
     } else {
         AttnArgs a{};
@@ -1100,6 +1102,7 @@ void Engine::encode_drafter(uint32_t set, const Plan& p, uint32_t rows) {
     io.n_tiles = p.tiles;
     io.ctiles = st.in<uint32_t>(st.o_ctiles);
     io.n_ctiles = p.chunked ? p.ctiles : 0;
+    io.ckey_blocks = p.ckey_blocks;
     io.cpos = dr.cpos.as<uint32_t>();
     io.keys_per_split = p.keys_per_split;
     io.max_splits = p.max_splits;

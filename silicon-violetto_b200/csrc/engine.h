@@ -59,6 +59,7 @@ struct Plan {
     bool verified = false;  // some run is a verified one of several rows
     bool head_all = false;  // every row of the step goes through the head, in order
     uint32_t ctiles = 0;   // chunk tiles of at most 64 rows (the prefill attention's blocks)
+    uint32_t ckey_blocks = 0;  // the blocks of 64 keys they see, summed
     bool chunked = false;  // some run is longer than VERIFY_T rows: the step's attention is the chunk kernel (encode.rs:299-355)
     uint32_t keys_per_split = 0, max_splits = 1;  // the attention's key split
     uint32_t max_keys = 0;                        // the longest run's keys
@@ -346,7 +347,7 @@ class Engine {
         uint32_t window;       // 0: every key; else the tiles' last `window` keys, extended down to a page boundary (the split kernel only)
         const uint32_t *meta, *tin, *tiles, *vis;
         const uint32_t* ctiles;  // chunk tiles, if the step's attention is the chunk kernel (n_ctiles > 0)
-        uint32_t n_ctiles;
+        uint32_t n_ctiles, ckey_blocks;
         bool kv_only;          // stop after the qkv projection has written K/V into the cache (the drafter's catch-up pass: a one-layer drafter's K/V depend on nothing after it)
         bool h_ready;          // the GEMM before this layer left bf16(h) in h_b and its sums of squares in ssq: no row pass before qkv
         const uint32_t* cpos;  // optional, per token: the cache position its K/V go to (NO_TOK: nowhere); NULL: its run's first position + its row

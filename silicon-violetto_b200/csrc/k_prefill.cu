@@ -8,11 +8,11 @@
 // 16 rows), walks the keys in blocks of 64 (four pages of K and of V by TMA into a three-stage ring of 128-byte-swizzled
 // shared memory, shared by the four warps; the G heads of a kv head find the same pages in L2), and keeps the whole
 // softmax online in registers: S = Q K^T lands in the accumulator layout that is the A-fragment layout of the next
-// product, so P goes into O += P V without leaving the registers. Two such groups of warps hold the same rows and take the
-// key blocks in turn, each with a ring of its own, and add up in shared memory at the end: a portion of 512 rows is 256
-// blocks, 1.7 an SM, and with four warps each the dependent chain of a key block was what the SM waited on. Two blocks of
-// eight warps still share an SM (128 registers, 97 KB). No partials and no merge kernel: the block writes the normalised
-// rows, fp32 and bf16.
+// product, so P goes into O += P V without leaving the registers. Where it pays (launch_attn_chunk), two such groups of warps
+// hold the same rows and take the key blocks in turn, each with a ring of its own, and add up in shared memory at the end: a
+// portion of 512 rows is 256 blocks, 1.7 an SM, and with four warps each the dependent chain of a key block is what the SM
+// waits on. Three blocks of one group share an SM (168 registers, 49 KB), or two of two groups (128 registers and 20 bytes
+// spilled, 97 KB). No partials and no merge kernel: the block writes the normalised rows, fp32 and bf16.
 //
 // The step's own rows are in the cache already (the qkv projection's epilogue wrote them), so every key is read from
 // there; what a row may see is the decode kernel's rule, per row: every cached key below the first position of its
@@ -28,7 +28,7 @@ namespace vlt {
 
 namespace prefill {
 
-constexpr uint32_t CQ = 64, CK = 64, HD = 64, PAGE = 16, WARPS = 4, GROUPS = 2, STAGES = 3;
+constexpr uint32_t CQ = 64, CK = 64, HD = 64, PAGE = 16, WARPS = 4, STAGES = 3;
 constexpr uint32_t STAGE_BYTES = 2 * CK * HD * 2;  // K block then V block
 constexpr uint32_t SPIN_LIMIT = 1u << 24;
 
@@ -49,12 +49,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x
                  "r"(y), "r"(bar)
                  : "memory");
 }
+template <uint32_t GROUPS>
 __device__ __forceinline__ void group_sync(uint32_t grp) {  // (constant barrier numbers: a variable one would claim all sixteen)
-    if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
+    if (GROUPS == 1) __syncthreads();
+    else if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
     else asm volatile("bar.sync 2, %0;" ::"n"(WARPS * 32) : "memory");
 }
+constexpr uint32_t blocks_per_sm(uint32_t groups) { return groups == 1 ? 3 : 2; }
 // grid (chunk tiles, query heads), GROUPS * 128 threads.
-__global__ void __launch_bounds__(GROUPS * WARPS * 32, 2) attn_chunk_kernel(ChunkAttnArgs a, const __grid_constant__ AttnMaps maps) {
+template <uint32_t GROUPS>
+__global__ void __launch_bounds__(GROUPS * WARPS * 32, blocks_per_sm(GROUPS)) attn_chunk_kernel(ChunkAttnArgs a, const __grid_constant__ AttnMaps maps) {
     pdl_start();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));  // the swizzle is a function of address bits 4..9
@@ -62,7 +66,7 @@ __global__ void __launch_bounds__(GROUPS * WARPS * 32, 2) attn_chunk_kernel(Chun
     __shared__ uint32_t fail[GROUPS];
 
     const uint32_t tile = blockIdx.x, h = blockIdx.y, kvh = h / (a.n_heads / a.kv.n_kv);
-    const uint32_t grp = threadIdx.x / (WARPS * 32), tid = threadIdx.x % (WARPS * 32), warp = tid / 32, lane = tid % 32, g = lane >> 2, tq = lane & 3;
+    const uint32_t grp = GROUPS == 1 ? 0 : threadIdx.x / (WARPS * 32), tid = GROUPS == 1 ? threadIdx.x : threadIdx.x % (WARPS * 32), warp = tid / 32, lane = tid % 32, g = lane >> 2, tq = lane & 3;
     uint8_t* ring = smem + grp * STAGES * STAGE_BYTES;
     uint64_t* bars = bars_all[grp];
     const uint32_t t0 = a.ctiles[2 * tile], rows = a.ctiles[2 * tile + 1];
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(GROUPS * WARPS * 32, 2) attn_chunk_kernel(Chun
                 }
             }
         }
-        group_sync(grp);  // every warp of the group is done with this stage
+        group_sync<GROUPS>(grp);  // every warp of the group is done with this stage
         if (fail[grp]) break;
         if (tid == 0 && i + STAGES < my_blocks) issue(i + STAGES);
     }
@@ -286,12 +290,27 @@ __global__ void __launch_bounds__(GROUPS * WARPS * 32, 2) attn_chunk_kernel(Chun
 
 }  // namespace prefill
 
-void launch_attn_chunk(const ChunkAttnArgs& a, cudaStream_t s) {
-    if (!a.n_ctiles) return;
-    const size_t smem = size_t(prefill::GROUPS) * prefill::STAGES * prefill::STAGE_BYTES + 1024;
+template <uint32_t GROUPS>
+static void launch_chunk_groups(const ChunkAttnArgs& a, cudaStream_t s) {
+    const size_t smem = size_t(GROUPS) * prefill::STAGES * prefill::STAGE_BYTES + 1024;
     static PerDevice configured;
-    configured.once([smem] { VLT_CUDA(cudaFuncSetAttribute(prefill::attn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); });
-    launch_pdl(prefill::attn_chunk_kernel, dim3(a.n_ctiles, a.n_heads), prefill::GROUPS * prefill::WARPS * 32, smem, s, a, *a.maps);
+    configured.once([smem] { VLT_CUDA(cudaFuncSetAttribute(prefill::attn_chunk_kernel<GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); });
+    launch_pdl(prefill::attn_chunk_kernel<GROUPS>, dim3(a.n_ctiles, a.n_heads), GROUPS * prefill::WARPS * 32, smem, s, a, *a.maps);
+}
+
+// key_blocks: the 64-key blocks of all the tiles together. Two groups of warps a block halve a tile's chain of key blocks, and
+// cost an exchange and a block less on the SM: they pay from four key blocks a tile on, unless they make a wave of blocks
+// more, and where every block has an SM to itself as soon as the second group has something to do (one key block and a
+// half a tile). Measured over 1 to 16 tiles of 32 heads and 1 to 40 key blocks a tile (one group / two, us): 1 tile, 1 key block
+// 10.3 / 10.4, 32: 51 / 38; 117 rows (2 tiles) 12.2 / 11.3; 8 tiles, 1 key block 11.8 / 13.3, 4: 16.4 / 16.3, 32: 60 / 48;
+// 12 tiles (384 blocks: one wave or two), 32 key blocks 68 / 78; 16 tiles (512: two waves either way), 1 key block
+// 18.5 / 20.5, 32: 117 / 87; 60 runs of 16 rows, 1 key block 29 / 43. The rule takes the faster one there, or one within 5 %.
+void launch_attn_chunk(const ChunkAttnArgs& a, uint32_t key_blocks, uint32_t sm_count, cudaStream_t s) {
+    if (!a.n_ctiles) return;
+    const uint32_t blocks = a.n_ctiles * a.n_heads;
+    auto waves = [&](uint32_t groups) { return (blocks + prefill::blocks_per_sm(groups) * sm_count - 1) / (prefill::blocks_per_sm(groups) * sm_count); };
+    if (2 * key_blocks >= (blocks <= sm_count ? 3 : 8) * a.n_ctiles && waves(2) <= waves(1)) launch_chunk_groups<2>(a, s);
+    else launch_chunk_groups<1>(a, s);
 }
 
 }  // namespace vlt

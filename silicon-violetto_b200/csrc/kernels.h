@@ -160,7 +160,7 @@ struct ChunkAttnArgs {
     float* out;
     uint16_t* out_b;
 };
-void launch_attn_chunk(const ChunkAttnArgs& a, cudaStream_t s);
+void launch_attn_chunk(const ChunkAttnArgs& a, uint32_t key_blocks, uint32_t sm_count, cudaStream_t s);  // key_blocks: the blocks of 64 keys that the tiles see, summed
 
 // The chain drafter's own kernels (k_draft.cu): inputs of the catch-up pass and of a draft pass, the
 // carried tap, and the argmax pick into feed / tree.

@@ -93,14 +93,16 @@ def test_a_computed_context_at_the_1b_dimensions_matches_the_oracle(tmp_path):
     prod.close()
 
 
-# Edges of a 64-key block and of the pair of key groups that share a chunk tile's blocks (9 .. 193 rows: one to four blocks,
-# odd counts leave the second group one less, a single block leaves it none), and of the GEMM's token blocks (two of 129 to
-# 256 tokens from 257 on, three from 513, four at 800; the last one short by up to its padding).
-@pytest.mark.parametrize("rows", [9, 64, 65, 128, 129, 193, 257, 272, 289, 511, 512, 513, 800])
-def test_a_chunk_at_the_edges_of_key_and_token_blocks_matches_the_oracle(rows):
+# Edges of a 64-key block, of the choice between one and two groups of warps a block (one key block and a half a tile on
+# average, from 65 rows on, where every block has an SM to itself; one group in all the steps counted for a single SM), of the
+# pair's shares (an odd count of key blocks leaves the second group one less), and of the GEMM's token blocks (two of 129 to 256
+# tokens from 257 on, three from 513, four at 800; the last one short by up to its padding).
+@pytest.mark.parametrize("sms", [0, 1])
+@pytest.mark.parametrize("rows", [9, 64, 65, 128, 129, 193, 257, 272, 289, 384, 385, 448, 511, 512, 513, 800])
+def test_a_chunk_at_the_edges_of_key_and_token_blocks_matches_the_oracle(rows, sms):
     w = util.weights("micro4", 0)
     kw = dict(max_seqs=1, max_step_tokens=rows + 37, max_chunk=rows + 37, max_seq_len=2 * rows + 64, max_head_rows=rows + 37)
-    prod = E.Engine(w, E.EngineConfig(global_kv_tokens=2 * rows + 64, **kw))
+    prod = E.Engine(w, E.EngineConfig(global_kv_tokens=2 * rows + 64, **kw), E.Tuning(sm_count=sms))
     orc = oracle.Engine(w, kv_tokens=2 * rows + 64, **kw)
     a = prod.new_seq()
     assert orc.new_seq() == a
@@ -114,5 +116,26 @@ def test_a_chunk_at_the_edges_of_key_and_token_blocks_matches_the_oracle(rows):
         want = orc.array("logits").reshape(-1, vocab)
         assert float(np.abs(out.logits - want).max()) <= TOL[0]
         same_state(prod, orc, 1, rows)
+    _caches_agree(prod, orc)
+    prod.close()
+
+
+def test_a_short_run_beside_a_long_one_leaves_the_second_group_of_warps_nothing():
+    """512 rows over 128 cached keys (eight tiles of three to ten key blocks) with a run of 9 rows and one of 70 beside them: two
+    groups of warps a block by the average, but one key block for the short run's tile, and a tile of six rows."""
+    w = util.weights("micro4", 0)
+    kw = dict(max_seqs=3, max_step_tokens=640, max_chunk=640, max_seq_len=800, max_head_rows=640)
+    prod = E.Engine(w, E.EngineConfig(global_kv_tokens=3 * 800, **kw))
+    orc = oracle.Engine(w, kv_tokens=3 * 800, **kw)
+    seqs = [prod.new_seq() for _ in range(3)]
+    assert [orc.new_seq() for _ in range(3)] == seqs
+    rng = np.random.default_rng(21)
+    vocab = prod.desc.vocab
+    for counts in ((128, 1, 60), (512, 9, 70)):  # (cached keys first)
+        runs = [(s, rng.integers(0, vocab, n).astype(np.uint32), E.Rows.ALL, False) for s, n in zip(seqs, counts)]
+        out = prod.debug_step(runs, E.StepOptions(read_logits=True))
+        orc.step(runs)
+        assert float(np.abs(out.logits - orc.array("logits").reshape(-1, vocab)).max()) <= TOL[0]
+        same_state(prod, orc, 3, sum(counts))
     _caches_agree(prod, orc)
     prod.close()
