@@ -44,7 +44,9 @@ __device__ __forceinline__ void cvt_i8x4(uint32_t w, uint32_t& lo, uint32_t& hi)
     hi = __byte_perm(__float_as_uint(f2), __float_as_uint(f3), 0x7632);
 }
 
-typedef GemmMapPair Maps;
+struct Maps {
+    TensorMap a, b;
+};
 
 struct Args {
     MatArgs m;
@@ -588,7 +590,7 @@ void launch_gemm(const MatArgs& a, GemmMaps& maps, uint32_t sm_count, uint32_t* 
     static PerDevice configured;
     // The MMA's N is at most 256 tokens: a longer step goes in equal blocks of at most that many.
     const uint32_t n_blocks = (a.n + 255) / 256, n_pad = ((a.n + n_blocks - 1) / n_blocks + 15) / 16 * 16, n_rows = (a.n + 15) / 16 * 16;
-    const gemm::Maps& pair = maps.get(a.W, a.Xb, a.m, a.k, a.int8, n_rows, n_pad);
+    const gemm::Maps pair{maps.weights(a.W, a.m, a.k, a.int8), maps.tokens(a.Xb, a.k, n_rows, n_pad)};
     // Shared memory: B stages of n_pad x 128 B; bf16 weights, as many A stages of 16 KiB; int8 weights, A
     // stages in tensor memory behind the accumulator and raw stages of 8 KiB in the shared memory left.
     const uint32_t a_bytes = gemm::BM * gemm::BK * 2, b_bytes = n_pad * gemm::BK * 2, raw_bytes = gemm::BM * gemm::BK;

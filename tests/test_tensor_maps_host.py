@@ -39,7 +39,7 @@ def test_weights_of_the_other_type_at_the_same_address_get_a_map_of_their_own(tm
     const bool first = {first};
     for (int round = 0; round < 2; round++)
         for (const bool int8 : {{first, !first}}) {{
-            const Asked a = asked(maps.get(w, x, 256, 512, int8, 48, 48).a), b = asked(maps.get(w, x, 256, 512, int8, 48, 48).b);
+            const Asked a = asked(maps.weights(w, 256, 512, int8).bytes), b = asked(maps.tokens(x, 512, 48, 48).bytes);
             assert(a.base == w && a.inner == 512 && a.rows == 256 && a.box_inner == 64 && a.box_rows == 128);
             assert(a.elem == (int8 ? 1u : 2u) && a.s128 == !int8 && a.s64 == int8);
             assert(b.base == x && b.inner == 512 && b.rows == 48 && b.box_inner == 64 && b.box_rows == 48 && b.elem == 2 && b.s128 && !b.s64);
@@ -52,6 +52,16 @@ def test_maps_follow_every_size_of_both_operands(tmp_path):
         for (uint32_t k : {64u, 512u})
             for (uint32_t rows : {16u, 272u, 288u})
                 for (uint32_t pad : {16u, 144u}) {
-                    const Asked a = asked(maps.get(w, x, m, k, true, rows, pad).a), b = asked(maps.get(w, x, m, k, true, rows, pad).b);
+                    const Asked a = asked(maps.weights(w, m, k, true).bytes), b = asked(maps.tokens(x, k, rows, pad).bytes);
                     assert(a.rows == m && a.inner == k && b.inner == k && b.rows == rows && b.box_rows == pad);
                 }""")
+
+
+def test_a_step_of_another_length_makes_one_map_for_each_buffer_of_tokens_and_none_for_the_weights(tmp_path):
+    run(tmp_path, """
+    for (uint32_t n = 16; n <= 512; n += 16)
+        for (int layer = 0; layer < 16; layer++) {
+            maps.weights(buf + layer, 256, 512, true);
+            maps.tokens(x, 512, n, n <= 256 ? n : (n / 2 + 15) / 16 * 16);
+        }
+    assert(made == 16 + 32);""")
