@@ -10,6 +10,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace vlt {
@@ -34,7 +35,8 @@ inline std::atomic<uint64_t>& launch_counter() {
 
 // Work that must happen once per CUDA device (cudaFuncSetAttribute applies to the current device only, and one
 // process may hold engines on several devices): `once(f)` runs f the first time it is called with a given device
-// current, under a lock, so that a second thread on the same device waits for the set-up instead of racing it.
+// current, under a lock, so that a second thread on the same device waits for the set-up instead of racing it. A set-up that
+// fails (f throws, or returns a false value where the caller must not see exceptions) is tried again by the next call.
 class PerDevice {
   public:
     template <typename F>
@@ -43,7 +45,8 @@ class PerDevice {
         if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
         std::lock_guard<std::mutex> lock(mu_);
         if ((done_ >> dev) & 1ull) return;
-        f();
+        if constexpr (std::is_void_v<decltype(f())>) f();
+        else if (!f()) return;
         done_ |= 1ull << dev;
     }
 

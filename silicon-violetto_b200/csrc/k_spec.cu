@@ -389,6 +389,7 @@ cudaError_t launch_spec_accept(const uint16_t* p, const uint16_t* q, const uint3
     configured.once([&] {
         e = cudaFuncSetAttribute(stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(STAGE_MAX));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(decide_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(2 * STAGE_MAX));
+        return e == cudaSuccess;
     });
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
