@@ -560,7 +560,7 @@ def folder_figure(E, local, c, files, work, steps, stream_counts, hbm_peak, tc_p
 
 def prefill_figure(E, path, ctx, local, chunk=512):
     """A `ctx`-token prompt of the reference's LCG ids computed in chunks of `chunk` tokens through the generator (the
-    tensor-core GEMM in blocks of 256 tokens, the chunk attention kernel), one stream; device time from the first chunk's
+    tensor-core GEMM in blocks of at most 256 tokens, the chunk attention kernel), one stream; device time from the first chunk's
     start to the last one's end."""
     from silicon_violetto_b200 import synth
     cfg = E.EngineConfig(max_seqs=1, max_step_tokens=chunk, max_chunk=chunk, global_kv_tokens=ctx + 64, max_seq_len=ctx + 64, max_head_rows=8, device_ordinal=local)

@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(threads_of(CONV_WARPS), CONV_WARPS == 16 ? 1 :
 
 typedef void (*GemmEntry)(const gemm::Maps, const gemm::Args);
 static GemmEntry gemm_entry(bool int8, uint32_t epi, bool paired = false) {
-    if (paired) return gemm::gemm_kernel<true, EPI_HEAD, 8>;  // the only shape that runs in waves
+    if (paired) return gemm::gemm_kernel<true, EPI_HEAD, 8>;  // the head over the vocabulary (launch_gemm says when)
     switch (epi) {
     case EPI_NORM: return int8 ? gemm::gemm_kernel<true, EPI_NORM> : gemm::gemm_kernel<false, EPI_NORM>;
     case EPI_RESID: return int8 ? gemm::gemm_kernel<true, EPI_RESID> : gemm::gemm_kernel<false, EPI_RESID>;

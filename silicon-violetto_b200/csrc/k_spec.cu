@@ -130,10 +130,10 @@ __device__ __forceinline__ float row_max(const RowWork& w) {
 // are the halves of packed registers; the maximum is taken on packed bf16, whoever's ids they are. What the cluster has to
 // agree on is the maximum alone: every block stores its own into the others, which a first cluster barrier, under way while the
 // row comes in, knows to have started, and a second one says that the maxima are there.
-// What bounds it: a row's 256 KiB of shared memory let 131 rows run at a time, and such a wave takes 5 us of HBM, 5 us of the
-// fp32 pipe (11 packed operations for two ids) and a barrier one after another. Three kernels without clusters that read the
-// row twice (maxima; sums; decision) took 24 / 67 us with the decision at 18 / 288 rows of 128 256 ids, one block per row
-// 73 / 122, this 21 / 62.
+// What bounds it: at 128 256 ids a block takes 33 KB, six fit an SM and 104 rows run at a time; a wave of them loads, finds its
+// maxima and adds up one after another, and 288 rows are three waves (43 us alone: issue slots 57 % active, DRAM 21 %). Three
+// kernels without clusters that read the row twice (maxima; sums; decision) took 24 / 67 us with the decision for 1 / 32
+// streams of k = 4 (9 / 288 rows), one block per row 73 / 122, this 22 / 62.
 constexpr uint32_t STATS_THREADS = SC_THREADS / 2;
 template <bool STAGED>
 __global__ void __cluster_dims__(SC_CTAS, 1, 1) __launch_bounds__(STATS_THREADS) stats_kernel(const uint16_t* __restrict__ p, const uint16_t* __restrict__ q,

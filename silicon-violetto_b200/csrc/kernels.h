@@ -231,8 +231,8 @@ void launch_limite_compact(const RunIn* runs, const uint32_t* path, const uint32
                            uint16_t* k_global, uint16_t* v_global, const LimiteKv& local, const LimiteKv& global, uint32_t n_local, uint32_t n_global, uint32_t n_runs,
                            cudaStream_t s);
 
-// The tcgen05 GEMM for 16..256 tokens: needs Xb (bf16 X, rows padded to 16), inv_in for the
-// normed epilogues, m a multiple of 128, one int8 scale per row.
+// The tcgen05 GEMM for any number of tokens (in blocks of at most 256): needs Xb (bf16 X, rows padded to 16), inv_in or ssq_in
+// for the normed epilogues, m a multiple of 128 and k of 64; int8 with one scale per row or in groups of a power of two from 8.
 bool gemm_supported(const MatArgs& a);
 void launch_gemm(const MatArgs& a, GemmMaps& maps, uint32_t sm_count, uint32_t* err_flag, cudaStream_t s, bool allow_paired = true);
 void launch_matmul_stream(const MatArgs& a, uint32_t sm_count, cudaStream_t s);  // n <= 8, tensor cores fed from registers

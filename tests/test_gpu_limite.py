@@ -287,7 +287,7 @@ def test_limite_int8_scale_groups_through_the_gemm(tmp_path, group):
 
 
 def test_limite_step_longer_than_a_gemm_launch(tmp_path):
-    """Ten streams' prompt chunks of 32 rows in one step of 320 tokens: the GEMMs run in blocks of 256 and 64 tokens (the
+    """Ten streams' prompt chunks of 32 rows in one step of 320 tokens: the GEMMs run in two blocks of 160 tokens (the
     bf16 inputs and sums of squares a layer's last projection leaves for the next are indexed by the step's token, not
     the block's), the attention in 40 tiles of 8 rows; then all ten decode."""
     path = tmp_path / "limite_wide.vlt"

@@ -1,4 +1,4 @@
-"""Chunked prefill: prompt chunks of hundreds of rows through the tensor-core GEMM in blocks of 256 tokens and the chunk
+"""Chunked prefill: prompt chunks of hundreds of rows through the tensor-core GEMM in equal blocks of at most 256 tokens and the chunk
 attention kernel (rows as the MMA's M side, keys read once per 64 rows), against the oracle: logits, the K/V the chunks
 leave in the cache, and every integer of the step state. Steps that mix a prompt chunk with decode and verify runs of
 other sequences (continuous batching) take the same kernel."""
@@ -50,7 +50,7 @@ def test_prompt_chunks_match_the_oracle(name, int8_group):
         same_state(prod, orc, n_runs, n)
         return err
 
-    # A 300-row chunk (two GEMM blocks: 256 + 44 tokens; five chunk tiles), every 37th-ish row through the head via a second run.
+    # A 300-row chunk (317 tokens: two GEMM blocks of 160, the second short by three; six chunk tiles), every 37th-ish row through the head via a second run.
     e1 = step([(seqs[0], prompt[:300], E.Rows.LAST, False), (seqs[1], prompt[300:317], E.Rows.ALL, False)], 2, 317)
     # Then a step that mixes: the next chunk of sequence 0 (attends 300 cached keys + itself), a one-token decode run of
     # sequence 1, and a verify run of sequence 2 over a small draft tree after its own short prefill.
