@@ -217,6 +217,7 @@ Engine::Engine(const std::string& weights, const EngineConfig& c, const Tuning& 
             lim->gates.alloc(n * md.n_heads * 4, false);
             lim->part.alloc(n * md.n_heads * size_t(LIMITE_MAX_SPLITS) * LIMITE_PART * 4, false);
         }
+        if (!model.limite) init_decode();
         VLT_CUDA(cudaDeviceSynchronize());
     }
 }
@@ -415,6 +416,7 @@ Plan Engine::plan(uint32_t set, const std::vector<PlanRun>& runs, Rows hidden) {
         max_count = std::max(max_count, count);
         p.branches = p.branches || (run.verify && count > 2);
         p.verified = p.verified || (run.verify && count > 1);
+        if (ri < 8) p.cached[ri] = sq.len;
         sq.len = new_len;
     }
     if (head_rows.size() > cfg.max_head_rows) throw Error(std::to_string(head_rows.size()) + " head rows (max " + std::to_string(cfg.max_head_rows) + ")");
@@ -733,7 +735,7 @@ void Engine::encode_sample(uint32_t set, uint32_t rows) {
 }
 
 // engine/src/engine/encode.rs:383-412 `encode_tail`.
-void Engine::encode_tail(uint32_t set, const Plan& p) {
+void Engine::encode_tail(uint32_t set, const Plan& p, bool have_logits) {
     StepSet& st = sets[set];
     const ModelDesc& md = model.md;
     const float* h = s.h.as<float>();
@@ -741,7 +743,9 @@ void Engine::encode_tail(uint32_t set, const Plan& p) {
     SpecStepArgs sa{};
     if (p.n_hidden) launch_prep_rows(h, st.in<uint32_t>(st.o_hidden_rows), p.n_hidden, md.d, md.eps, s.hfin_all.as<float>(), nullptr, nullptr, true, false, stream);
     if (p.n_head && !(skip & 256)) {
-        if (use_gemm(model.head, p.n_head) && p.head_all && !(skip & 64) && layer_carries(model.layers.back(), p.n)) {
+        if (have_logits) {
+            // (the layers' launch took the head along)
+        } else if (use_gemm(model.head, p.n_head) && p.head_all && !(skip & 64) && layer_carries(model.layers.back(), p.n)) {
             // Every row goes through the head (a verify step): the last down projection left bf16(h) and the sums of squares.
             matmul_gemm(model.head, p.n_head, s.h_b.as<uint16_t>(), s.logits.as<float>(), nullptr, EPI_HEAD, nullptr, nullptr, 0, nullptr, nullptr, s.ssq.as<float>());
         } else if (use_gemm(model.head, p.n_head)) {
@@ -792,6 +796,108 @@ void Engine::encode_tail(uint32_t set, const Plan& p) {
         launch_kv_compact(st.in<RunIn>(st.o_runs), s.path.as<uint32_t>(), s.path_len.as<uint32_t>(), s.lens.as<uint32_t>(), kv.k.as<uint16_t>(),
                           kv.v.as<uint16_t>(), kv.page_table.as<uint32_t>(), kv_args(), p.n_runs, md.n_layers, stream);
 }
+
+void Engine::init_decode() {
+    const ModelDesc& md = model.md;
+    int device_sms = 0, together = 0;
+    VLT_CUDA(cudaDeviceGetAttribute(&device_sms, cudaDevAttrMultiProcessorCount, cfg.device));
+    VLT_CUDA(cudaDeviceGetAttribute(&together, cudaDevAttrCooperativeLaunch, cfg.device));
+    if (!together || sm_count > uint32_t(device_sms) || !decode_fits(md, model.layers, sm_count)) return;
+    std::vector<DecodeMap> maps;
+    std::vector<const uint16_t*> scales;
+    auto put = [&](const Matrix& m) {
+        maps.emplace_back();
+        decode_map(&maps.back(), m);
+        scales.push_back(m.scales);
+    };
+    for (const Layer& l : model.layers)
+        for (const Matrix* m : {&l.qkv, &l.o, &l.gate_up, &l.down}) put(*m);
+    if (decode_head_fits()) put(model.head);
+    dec.maps.alloc(maps.size() * sizeof(DecodeMap), false);
+    dec.maps.write_vec(0, maps);
+    dec.scales.alloc(scales.size() * sizeof(scales[0]), false);
+    dec.scales.write_vec(0, scales);
+    dec.most = std::min(8u, cfg.max_step_tokens);
+    const DecodeArena a = decode_arena(md, model.layers[0].qkv.int8, dec.most, decode_max_splits(md.n_kv, sm_count));
+    for (Buffer& b : dec.words) b.alloc(size_t(md.n_layers) * a.layer_bytes + a.q, false);
+    reset_decode();
+}
+
+void Engine::reset_decode() {
+    for (int i = 0; i < 2; i++) {
+        if (dec.words[i].dev) VLT_CUDA(cudaMemsetAsync(dec.words[i].dev, 0xff, dec.words[i].bytes, stream));
+        dec.used[i] = 0;
+    }
+}
+
+// Steps of at most 8 tokens whose runs are tiles of their own, unless a knob asks for one of the kernels it replaces. (Profiled
+// steps take the kernels apart: their groups cannot be told from within one launch.)
+bool Engine::use_decode(const Plan& p) const {
+    return p.n <= dec.most && p.tiles == p.n_runs && p.tiles * model.md.n_kv <= DECODE_UNITS * sm_count && !p.chunked && !skip && !profile && !tuning.plain_attention && !tuning.attn_keys_per_cta && !tuning.gemm_min_rows;
+}
+
+void Engine::encode_decode(uint32_t set, const Plan& p) {
+    StepSet& st = sets[set];
+    const ModelDesc& md = model.md;
+    const Layer& first = model.layers[0];
+    DecodeArgs a{};
+    a.maps = dec.maps.as<DecodeMap>();
+    a.scales = dec.scales.as<const uint16_t*>();
+    a.n_layers = md.n_layers;
+    a.n = p.n;
+    a.n_tiles = p.tiles;
+    a.d = md.d;
+    a.ffn = md.ffn;
+    a.n_heads = md.n_heads;
+    a.kv = kv_args();
+    decode_split(a, p.cached, sm_count);
+    a.eps = md.eps;
+    a.scale_log2 = md.attn_scale * 1.44269504088896340736f;
+    a.meta = s.meta.as<uint32_t>();
+    a.tiles = st.in<uint32_t>(st.o_tiles);
+    a.vis = st.in<uint32_t>(st.o_vis);
+    a.page_table = kv.page_table.as<uint32_t>();
+    a.rope = rope_tab.as<float>();
+    a.k_cache = kv.k.as<uint16_t>();
+    a.v_cache = kv.v.as<uint16_t>();
+    a.h = s.h.as<float>();
+    a.ar = decode_arena(md, first.qkv.int8, p.n, a.max_splits);
+    a.err_flag = s.err_flag.as<uint32_t>();
+    // A launch ends behind each tapped layer: the tap is a row pass over its output.
+    for (uint32_t l0 = 0, l1; l0 < md.n_layers; l0 = l1) {
+        l1 = md.n_layers;
+        for (uint32_t t : tap_layers)
+            if (t >= l0 && t + 1 < l1) l1 = t + 1;
+        a.l0 = l0;
+        a.l1 = l1;
+        if (l1 == md.n_layers && decode_head(p)) {
+            a.head_s = model.head.scales;
+            a.head_rows = st.in<uint32_t>(st.o_head_rows);
+            a.logits = s.logits.as<float>();
+            a.n_head = p.n_head;
+            a.vocab = md.vocab;
+            a.vocab_real = md.vocab_real;
+        }
+        const uint32_t turn = dec.turn, other = turn ^ 1u;
+        a.arena = dec.words[turn].as<uint8_t>();
+        a.clear = dec.words[other].as<uint8_t>();
+        a.clear_bytes = dec.used[other];
+        launch_decode(a, attn_maps, first.qkv.int8, sm_count, stream);
+        dec.used[turn] = size_t(l1 - l0) * a.ar.layer_bytes + a.ar.q;
+        dec.used[other] = 0;
+        dec.turn = other;
+        auto tap = std::find(tap_layers.begin(), tap_layers.end(), l1 - 1);
+        if (tap != tap_layers.end())
+            launch_prep_rows(s.h.as<float>(), nullptr, p.n, md.d, md.eps, tap_bufs[tap - tap_layers.begin()].as<float>(), nullptr, nullptr, true, true, stream);
+    }
+}
+
+// Whether such a step's launch takes the head along: of the layers' type, whole tiles of rows, one scale a row.
+bool Engine::decode_head_fits() const {
+    const Matrix& h = model.head;
+    return h.int8 == model.layers[0].qkv.int8 && (!h.int8 || h.group == h.k) && h.m % 16 == 0 && !h.bias && !(reinterpret_cast<uintptr_t>(h.w) % 16) && !(reinterpret_cast<uintptr_t>(h.scales) % 16);
+}
+bool Engine::decode_head(const Plan& p) const { return p.n_head && p.n_head <= 8 && decode_head_fits(); }
 
 // The reference's own architecture, encode.rs:99-192 `encode_forward` / `encode_layer` and :383-412 `encode_tail`: the
 // layers' extras are k_limite.cu's kernels, the projections the streamed matmul with the matrix scales and residual
@@ -911,9 +1017,12 @@ void Engine::encode_forward(uint32_t set, const Plan& p) {
     if (model.layered) { encode_forward_layered(set, p); return; }
     if (model.limite) { encode_forward_limite(set, p); return; }
     begin_step(set, p);
-    for (uint32_t li = 0; li < model.md.n_layers; li++) encode_layer(set, p, li);
+    const bool whole = use_decode(p);
+    if (whole) encode_decode(set, p);
+    else
+        for (uint32_t li = 0; li < model.md.n_layers; li++) encode_layer(set, p, li);
     const int sp = span_begin(G_TAIL);
-    encode_tail(set, p);
+    encode_tail(set, p, whole && decode_head(p));
     span_end(sp);
 }
 
@@ -967,6 +1076,7 @@ void Engine::check_device_error(uint32_t set) {
     const uint32_t flag = *st.hout<uint32_t>(st.o_err);
     if (flag) {
         VLT_CUDA(cudaMemsetAsync(s.err_flag.dev, 0, 4, stream));
+        reset_decode();
         *st.hout<uint32_t>(st.o_err) = 0;
         throw Error("a kernel's bounded wait ran out (device error flag " + std::to_string(flag) + "): the step's results are not valid");
     }

@@ -54,6 +54,7 @@ struct PlanRun {
 
 // engine/src/engine/plan.rs:20-37.
 struct Plan {
+    uint32_t cached[8] = {};  // the first runs' lengths before the step
     uint32_t n = 0, n_head = 0, n_hidden = 0, n_runs = 0, tiles = 0, max_run = 0;
     bool branches = false;
     bool verified = false;  // some run is a verified one of several rows
@@ -225,6 +226,20 @@ class Engine {
     Buffer spec_p, spec_q, spec_small;  // spec_accept's device copies, grown on demand
     AttnMaps attn_maps;
     GemmMaps gemm_maps;  // of this engine's buffers
+    // k_decode.cu's: the layers' matrices, and the two sets of words that its launches take turns with (what the set's last launch
+    // left in it is cleared by the launch in between).
+    struct Decode {
+        Buffer maps, scales, words[2];
+        size_t used[2] = {0, 0};
+        uint32_t turn = 0;
+        uint32_t most = 0;  // tokens; 0: the model's sizes are not the kernel's
+    } dec;
+    void init_decode();
+    void reset_decode();  // after a wait that ran out
+    bool use_decode(const Plan& p) const;
+    bool decode_head_fits() const;
+    bool decode_head(const Plan& p) const;
+    void encode_decode(uint32_t set, const Plan& p);
     // The chain drafter (a benchmark extension; the reference's drafter.rs is a block drafter): fc over
     // (feature ; embedding), one decoder layer with a cache of its own on the target's page table, a head
     // over a draft vocabulary.
@@ -362,7 +377,7 @@ class Engine {
     void encode_layer(uint32_t set, const Plan& p, uint32_t li, bool capture = false);
     void encode_layer_io(const LayerIO& io, bool capture = false);
     StepOutput read_output(const Plan& p, const StepOptions& opts, double gpu_seconds);
-    void encode_tail(uint32_t set, const Plan& p);
+    void encode_tail(uint32_t set, const Plan& p, bool have_logits = false);  // have_logits: the head is done
     void encode_sample(uint32_t set, uint32_t rows);
     void attention_split(Plan& p, uint32_t max_keys, uint32_t n_tiles) const;
     const Buffer* named(const std::string& name, uint32_t* set_off, size_t* words) const;

@@ -354,6 +354,18 @@ void make_tensor_map_2d(void* out_map, const void* base, uint64_t inner, uint64_
     if (r != CUDA_SUCCESS) throw Error("cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
 }
 
+// A matrix of `rows` rows as [pieces of a row][rows][bytes of a piece], a box of 16 pieces of `box_rows` rows, 128-byte swizzled.
+void make_tensor_map_rows(void* out_map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t piece, uint32_t box_rows) {
+    static TmaEncoder enc;
+    const cuuint64_t dims[3] = {piece, rows, row_bytes / piece};
+    const cuuint64_t strides[2] = {row_bytes, piece};
+    const cuuint32_t box[3] = {piece, box_rows, 16};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc.fn(static_cast<CUtensorMap*>(out_map), CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw Error("cuTensorMapEncodeTiled failed with code " + std::to_string(int(r)));
+}
+
 // The K and V pools as [all layers' rows][64] bf16, a box of one page.
 void attn_maps_init(AttnMaps* m, const uint16_t* k_cache, const uint16_t* v_cache, uint64_t total_rows) {
     static_assert(sizeof(CUtensorMap) == sizeof(m->k), "tensor map size");

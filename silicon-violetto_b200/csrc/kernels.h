@@ -118,6 +118,7 @@ struct alignas(64) AttnMaps {
     alignas(64) uint8_t k[128];
     alignas(64) uint8_t v[128];
 };
+void make_tensor_map_rows(void* out_map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t piece, uint32_t box_rows);
 void attn_maps_init(AttnMaps* m, const uint16_t* k_cache, const uint16_t* v_cache, uint64_t total_rows);
 struct AttnArgs {
     const AttnMaps* maps;  // host pointer
@@ -143,6 +144,44 @@ struct AttnArgs {
 constexpr uint32_t ATTN_PART = 68;  // floats per partial: m, l, 2 pad, o[64]
 void launch_attn_mma(const AttnArgs& a, cudaStream_t s);
 void launch_attn_combine(const AttnArgs& a, cudaStream_t s);
+
+// The layers l0 .. l1 - 1 of a plain decoder's step of at most 8 tokens, and its head, in one launch (k_decode.cu).
+constexpr uint32_t DECODE_RESID_TILES = 4;    // row tiles of the residual stream a block may own
+constexpr uint32_t DECODE_UNITS = 8;          // units of the attention a block may have
+struct alignas(64) DecodeMap { alignas(64) uint8_t bytes[128]; };  // a matrix's tensor map
+struct DecodeArena {                          // where a layer's words lie (x1, its input, at 0), in bytes
+    uint32_t over, ss1, q, kvn, part, at, x2, ss2, act, layer_bytes;
+    uint32_t half_d, half_o, half_ffn;        // from rows in bf16 to the same in fp16
+};
+struct DecodeArgs {
+    const DecodeMap* maps;                    // [layer][qkv, o, gate_up, down], then the head's
+    const uint16_t* const* scales;            // the same (NULL: bf16)
+    uint32_t n_layers, l0, l1, n, n_tiles;              // tokens; attention tiles, one a run
+    uint32_t d, ffn, n_heads;
+    KvArgs kv;
+    uint32_t split_pages, max_splits, unit0[9];  // of the cached keys: pages a split, the most splits of a tile, a tile's first split
+    uint32_t n_units, heads_per_kv, per_kv_recip;  // units of the attention; query heads a kv head, and 65536 over that rounded up
+    float eps, scale_log2;
+    const uint32_t *meta, *tiles, *vis, *page_table;
+    const float* rope;
+    uint16_t *k_cache, *v_cache;
+    float* h;                                 // [n][d], in and out
+    uint8_t *arena, *clear;                   // this launch's words (all ones), and the other set, to be made so
+    size_t clear_bytes;
+    DecodeArena ar;
+    const uint16_t* head_s;                   // n_head > 0: the head of these rows as well
+    const uint32_t* head_rows;
+    float* logits;
+    uint32_t n_head, vocab, vocab_real;
+    uint32_t wbytes;                          // (launch_decode's)
+    uint32_t* err_flag;
+};
+bool decode_fits(const ModelDesc& md, const std::vector<Layer>& layers, uint32_t sm_count);
+inline uint32_t decode_max_splits(uint32_t n_kv, uint32_t sm_count) { return sm_count > n_kv ? sm_count / n_kv : 1u; }
+DecodeArena decode_arena(const ModelDesc& md, bool int8, uint32_t n, uint32_t max_splits);
+void decode_split(DecodeArgs& a, const uint32_t* cached, uint32_t sm_count);  // cached: each tile's keys before the step, at most
+void decode_map(DecodeMap* out, const Matrix& m);
+void launch_decode(DecodeArgs a, const AttnMaps& maps, bool int8, uint32_t sm_count, cudaStream_t s);
 
 // Chunk (prefill) attention, k_prefill.cu: blocks of 64 rows of one run x one query head over all the keys the rows see,
 // no key split; writes the normalised rows (fp32 and, optionally, bf16).
