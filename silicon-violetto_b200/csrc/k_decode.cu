@@ -49,7 +49,7 @@ struct DecodeSmem {
     float ssp[RES_WARPS][8];    // a warp's share of a token's sum of squares
     uint32_t mx[2][8];          // a token's largest magnitude (its bits), by turns
     float sc[RES_WARPS / 4][2][16];  // a team's rows' scales, by buffer
-    float ml[RES_WARPS][2][8];  // attention: a warp's maximum and sum per column
+    float mw[8][RES_WARPS];     // attention: a warp's maximum per column
     uint32_t tok_tile[8], tok_row[8], vis[8];
     uint32_t t0[8], rows[8], slot[8], p0[8];
     Unit unit[DECODE_UNITS];    // the block's
@@ -89,7 +89,8 @@ __device__ __forceinline__ Patience patience(const DecodeArgs& a, DecodeSmem& sm
 // The warp that fills the ring: a copy of 32 KiB a stage (an SM starts no more than one of its copies in some 70 cycles: a copy for
 // each of the 16 rows' pieces, 0.6 us a stage, bound everything else). It walks over the block's items -- (row tile, 2 KiB of k) or
 // (unit, 8 pages) -- in the order the others want them. Whatever a copy needs is at hand before its turn: the ring is deep in bytes,
-// not in time.
+// not in time. (Not done: a second warp that has L2 fetch the items 3, 7 or 15 behind the ring's. One stream's step went from 609 to
+// 656, 671 and 709 us: the words that the chain waits for queue behind what HBM then delivers.)
 __device__ __forceinline__ void ask(const DecodeArgs& a, const AttnMaps& maps, DecodeSmem& sm, uint32_t stages) {
     const uint32_t lane = threadIdx.x % 32;
     uint32_t item = 0;
@@ -196,25 +197,24 @@ __device__ __forceinline__ float scale_of(uint32_t ph) { return ph == PH_O ? 64.
 // A pair of values (bf16 word w) from every `step`-th of the lanes that hold eight values of a token between them, as one 16-byte
 // store by the first of them.
 template <bool INT8>
-__device__ __forceinline__ void publish(uint8_t* words, uint32_t half, size_t at, uint32_t w, float times, uint32_t step, bool mine) {
+__device__ __forceinline__ void publish(uint8_t* words, uint32_t half, uint32_t at, uint32_t w, float times, uint32_t step, bool mine) {
     uint4 v;
     v.x = w;
     v.y = __shfl_down_sync(0xffffffffu, w, step);
     v.z = __shfl_down_sync(0xffffffffu, w, 2 * step);
     v.w = __shfl_down_sync(0xffffffffu, w, 3 * step);
     if (!mine) return;
-    st_whole(words + at * 2, v);
-    if (INT8) st_whole(words + half + at * 2, make_uint4(bf16x2_to_f16x2(v.x, times), bf16x2_to_f16x2(v.y, times), bf16x2_to_f16x2(v.z, times), bf16x2_to_f16x2(v.w, times)));
+    words += size_t(at) * 2;
+    st_whole(words, v);
+    if (INT8) st_whole(words + half, make_uint4(bf16x2_to_f16x2(v.x, times), bf16x2_to_f16x2(v.y, times), bf16x2_to_f16x2(v.z, times), bf16x2_to_f16x2(v.w, times)));
 }
 
-// Rows of the residual stream, tile `at`, row r of token tok: for the matmul behind, and the tile's sum of squares.
-template <bool INT8>
-__device__ __forceinline__ void publish_resid(const DecodeArgs& a, uint8_t* x, float* ss, uint32_t at, uint32_t tok, uint32_t r, float y) {
+// The sum of squares of a tile's 16 rows (row r of token tok to a lane).
+__device__ __forceinline__ void tile_squares(const DecodeArgs& a, float* ss, uint32_t tile, uint32_t tok, uint32_t r, float y) {
     float q = y * y;
 #pragma unroll
     for (int o = 1; o < 16; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    if (tok < a.n && r == 0) st_word(ss + at * 8 + tok, q);
-    publish<INT8>(x, a.ar.half_d, size_t(tok) * a.d + at * 16 + r, pack_bf16(y, __shfl_down_sync(0xffffffffu, y, 1)), 1.0f, 2, tok < a.n && r % 8 == 0);
+    if (tok < a.n && r == 0) st_word(ss + tile * 8 + tok, q);
 }
 
 // A warp's operands of one 128-byte piece of k: two halves of 64 bytes, a lane 16 bytes of each.
@@ -234,33 +234,38 @@ struct Piece {
     }
 };
 
-// The sums of squares of the tokens' rows, tile by tile: this warp's share, in lanes 0 .. 7.
-__device__ __forceinline__ float squares(const DecodeArgs& a, DecodeSmem& sm, Ctx& c, const float* ss, uint32_t tok) {
-    const uint32_t tiles = a.d / 16;
-    Patience p = patience(a, sm);
-    float sum = 0.0f;
-#pragma unroll 1
-    for (uint32_t t0 = c.warp + 16 * (c.lane / 8); t0 < tiles; t0 += 128) {  // two at a time: 128 tiles in one turn
-        uint32_t v0, v1;
-        do {
-            v0 = ld_word(ss + t0 * 8 + tok);
-            v1 = t0 + 64 < tiles ? ld_word(ss + (t0 + 64) * 8 + tok) : 0u;
-        } while ((v0 == ABSENT || v1 == ABSENT) && !p.over());
-        sum += __uint_as_float(v0);
-        sum += __uint_as_float(v1);
+// The sums of squares of the tokens' rows: this warp's share of the tiles, four lanes to a token (of column lane % 8). The first 128
+// tiles' words are asked for before the activations are polled for, and are there when those are.
+struct Squares {
+    const float* at;
+    uint32_t tile, tiles, v0, v1;
+    __device__ __forceinline__ void ask() {
+        v0 = tile < tiles ? ld_word(at + tile * 8) : 0u;
+        v1 = tile + 64 < tiles ? ld_word(at + (tile + 64) * 8) : 0u;
     }
-    __syncwarp();
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    return sum;
-}
+    __device__ __forceinline__ float sum(Patience p) {
+        float s = 0.0f;
+#pragma unroll 1
+        for (;;) {
+            while ((v0 == ABSENT || v1 == ABSENT) && !p.over()) ask();
+            s += __uint_as_float(v0);
+            s += __uint_as_float(v1);
+            tile += 128;
+            if (tile >= tiles) break;
+            ask();
+        }
+        __syncwarp();
+        s += __shfl_xor_sync(0xffffffffu, s, 8);
+        return s + __shfl_xor_sync(0xffffffffu, s, 16);
+    }
+};
 
 // One matmul phase: the block's row tiles of a matrix against the activations x [token][k] (bf16, polled for), the epilogue by phase.
 // Columns past the tokens repeat the last one's (nothing reads their sums).
 template <bool INT8>
 __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm, uint8_t* stages, float* red, uint4* xs, Ctx& c, uint32_t layer, uint32_t ph, const uint8_t* words, const float* ss) {
     using P = Piece<INT8>;
-    constexpr uint32_t WB = P::WB, E = P::E, R = P::R, KS = E / 4, PARTS = INT8 ? 1 : 2, CHUNK = INT8 ? 2 : 4;  // a group's parts of a row; pieces whose operands a warp holds (32 registers)
+    constexpr uint32_t WB = P::WB, E = P::E, R = P::R, KS = E / 4, PARTS = INT8 ? 1 : 2, CHUNK = 2;  // a group's parts of a row; pieces whose operands a warp holds (at most 32 registers)
     const uint32_t k = width_of(a, ph), tiles = tiles_of(a, ph), first = first_tile(ph);
     if (first >= tiles) return;
     const uint32_t pieces = k * WB / RES_PIECE, parts = (pieces + 15) / 16;
@@ -272,7 +277,12 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
     const bool share = size == 1;  // every group needs all of the activations: a warp polls for a sixteenth
 
     res_sync();  // (the phase before is done with the buffers)
-
+    Squares sq{nullptr, c.warp + 16 * (c.lane / 8), ss ? a.d / 16 : 0u, 0u, 0u};
+    if (ss) {
+        const uint32_t tok = min(c.lane % 8, nx - 1);
+        sq.at = ss + (ph == PH_HEAD ? a.head_rows[tok] : tok);
+        sq.ask();
+    }
     if (share) {
 #pragma unroll 1
         for (uint32_t i = c.warp * PARTS; i < min((c.warp + 1) * PARTS, pieces); i++) {
@@ -294,8 +304,7 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
         }
     }
     if (ss) {
-        const uint32_t tok = min(c.lane % 8, nx - 1);
-        const float s = squares(a, sm, c, ss, ph == PH_HEAD ? a.head_rows[tok] : tok);
+        const float s = sq.sum(patience(a, sm));
         if (c.lane < 8) sm.ssp[c.warp][c.lane] = s;
     }
     if (share || ss) res_sync();
@@ -308,10 +317,10 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
     }
     float inv = 1.0f;
     if (ss) {
-        float sq = 0.0f;
-#pragma unroll 4
-        for (uint32_t w = 0; w < RES_WARPS; w++) sq += sm.ssp[w][2 * kq + c.lane / 16];
-        inv = rsqrtf(sq / float(a.d) + a.eps);
+        float sq = sm.ssp[c.lane % 16][2 * kq + c.lane / 16];
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        inv = rsqrtf(sq * a.inv_d + a.eps);
     }
     const uint32_t mine = (tiles - first + gridDim.x - 1) / gridDim.x;
     // Lane (g, t) reads 16 bytes of MMA row g, and of row g + 8, which are memory rows `row` and `row` + 8: rows four apart side by
@@ -429,10 +438,7 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
         sum *= inv;
         const float other = __shfl_xor_sync(0xffffffffu, sum, 1);  // the pair's other row
         uint8_t* ar = layer_arena(a, layer);
-        if (ph == PH_GU) {
-            const float y = sum * (1.0f / (1.0f + expf(-sum))) * other;  // (of the even rows)
-            publish<INT8>(ar + a.ar.act, a.ar.half_ffn, size_t(tok) * a.ffn + tile * 8 + r / 2, pack_bf16(y, __shfl_down_sync(0xffffffffu, y, 2)), scale_of(PH_DOWN), 4, tok < a.n && r == 0);
-        } else if (ph == PH_HEAD) {
+        if (ph == PH_HEAD) {
             const uint32_t at = tile * 16 + r;
             if (tok < a.n_head) a.logits[size_t(tok) * a.vocab + at] = at < a.vocab_real ? sum : -INFINITY;
         } else if (ph == PH_QKV) {
@@ -442,29 +448,41 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
                 float y0 = sum, y1 = other;
                 if (head < a.n_heads + a.kv.n_kv) {
                     const float2 cs = sm.cs[tok][pair];
-                    const float r0 = __fadd_rn(__fmul_rn(cs.x, y0), __fmul_rn(cs.y, y1)), r1 = __fsub_rn(__fmul_rn(cs.x, y1), __fmul_rn(cs.y, y0));
-                    y0 = r0;
-                    y1 = r1;
+                    y0 = __fadd_rn(__fmul_rn(cs.x, sum), __fmul_rn(cs.y, other));
+                    y1 = __fsub_rn(__fmul_rn(cs.x, other), __fmul_rn(cs.y, sum));
                 }
                 if (head < a.n_heads) {
-                    st_word(reinterpret_cast<uint32_t*>(ar + a.ar.q) + (tok * a.n_heads + head) * (HD / 2) + pair, pack_bf16(__fmul_rn(y0, a.scale_log2), __fmul_rn(y1, a.scale_log2)));
+                    st_word(ar + a.ar.q + ((tok * a.n_heads + head) * (HD / 2) + pair) * 4, pack_bf16(__fmul_rn(y0, a.scale_log2), __fmul_rn(y1, a.scale_log2)));
                 } else {
                     const bool is_v = head >= a.n_heads + a.kv.n_kv;
                     const uint32_t kvh = head - a.n_heads - (is_v ? a.kv.n_kv : 0), word = pack_bf16(y0, y1);
-                    st_word(reinterpret_cast<uint32_t*>(ar + a.ar.kvn) + ((tok * 2 + is_v) * a.kv.n_kv + kvh) * (HD / 2) + pair, word);
+                    st_word(ar + a.ar.kvn + (((tok * 2 + is_v) * a.kv.n_kv + kvh) * (HD / 2) + pair) * 4, word);
                     const size_t at = sm.kvrow[tok] + (size_t(layer) * a.kv.n_pages * a.kv.n_kv + kvh) * PAGE * HD;
                     reinterpret_cast<uint32_t*>((is_v ? a.v_cache : a.k_cache) + at)[pair] = word;
                 }
             }
         } else {
-            float& h = sm.resid[i_tile][tok][r];
-            const float y = h + sum;
-            h = y;
-            const bool out = ph == PH_DOWN && layer + 1 == a.l1;
-            if (out && tok < a.n) a.h[size_t(tok) * a.d + tile * 16 + r] = y;
-            // (what down leaves is the next layer's input, or the head's)
-            uint8_t* to = ph == PH_O ? ar + a.ar.x2 : ar + a.ar.layer_bytes;
-            if (!out || a.n_head) publish_resid<INT8>(a, to, reinterpret_cast<float*>(to + (ph == PH_O ? a.ar.ss2 - a.ar.x2 : a.ar.ss1)), tile, tok, r, y);
+            const bool gu = ph == PH_GU;
+            float y;
+            uint32_t to, at;  // where it goes: rows in the arena, and in them
+            if (gu) {
+                y = sum * __fdividef(1.0f, 1.0f + __expf(-sum)) * other;  // (of the even rows; the hardware's exponential and quotient: their errors are far below the rounding to bf16)
+                to = a.ar.act;
+                at = tok * a.ffn + tile * 8 + r / 2;
+            } else {
+                float& h = sm.resid[i_tile][tok][r];
+                h += sum;
+                y = h;
+                to = ph == PH_O ? a.ar.x2 : a.ar.layer_bytes;  // (what down leaves is the next layer's input, or the head's)
+                at = tok * a.d + tile * 16 + r;
+                if (ph == PH_DOWN && layer + 1 == a.l1) {
+                    if (tok < a.n) a.h[at] = y;
+                    if (!a.n_head) continue;
+                }
+                tile_squares(a, reinterpret_cast<float*>(ar + to + (ph == PH_O ? a.ar.ss2 - a.ar.x2 : a.ar.ss1)), tile, tok, r, y);
+            }
+            const uint32_t pair = gu ? 2 : 1;  // lanes from one value to the next
+            publish<INT8>(ar + to, gu ? a.ar.half_ffn : a.ar.half_d, at, pack_bf16(y, __shfl_down_sync(0xffffffffu, y, pair)), scale_of(gu ? PH_DOWN : PH_GU), 2 * pair, tok < a.n && r % (8 * pair) == 0);
         }
     }
     c.items += mine * parts;
@@ -609,102 +627,113 @@ __device__ __forceinline__ void attention_unit(const DecodeArgs& a, DecodeSmem& 
     }
     if (have && c.lane == 0) bar_arrive(smem_u32(&sm.empty[ring_stage(c.items + have - 1)]), 1);
     c.items += have;
-    // The key groups meet.
-    res_sync();  // (the buffers' readers before are done)
+    // The key groups meet: first their maxima, then what each has, scaled to the largest.
+    const uint32_t cc = 2 * c.t;
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+        if (c.g == 0) sm.mw[cc + e][c.warp] = kg < KG ? m_run[e] : -INFINITY;
+    res_sync();  // (the buffers' readers before are done, too)
     constexpr uint32_t OS = HD + 4;
-    static_assert(RES_WARPS * 8 * OS * 4 <= RES_RED * 4 + RES_X, "the warps' sums fit");  // (over the operands' buffer, which a phase only uses before its second meeting)
+    static_assert(RES_WARPS * 8 * OS * 4 <= RES_RED * 4 + RES_X, "the warps' sums fit");
     if (kg < KG) {
 #pragma unroll
         for (int e = 0; e < 2; e++) {
+            float mm = -INFINITY;  // over the warps of this n-tile: cw, cw + NT, ...; every eighth of them a lane
+#pragma unroll 1
+            for (uint32_t w = cw + c.g * NT; w < KG * NT; w += 8 * NT) mm = fmaxf(mm, sm.mw[cc + e][w]);
             float l = l_run[e];
-            l += __shfl_xor_sync(0xffffffffu, l, 4);
-            l += __shfl_xor_sync(0xffffffffu, l, 8);
-            l += __shfl_xor_sync(0xffffffffu, l, 16);
-            const uint32_t cc = 2 * c.t + e;
-            if (c.g == 0) {
-                sm.ml[c.warp][0][cc] = m_run[e];
-                sm.ml[c.warp][1][cc] = l;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+                l += __shfl_xor_sync(0xffffffffu, l, o);
             }
+            const float wt = m_run[e] == -INFINITY ? 0.0f : fast_exp2(m_run[e] - mm);
+            float* to = red + (c.warp * 8 + cc + e) * OS + c.g;
 #pragma unroll
             for (int dm = 0; dm < 4; dm++) {
-                float* o = red + (c.warp * 8 + cc) * OS + 16 * dm + c.g;
-                o[0] = oacc[dm][e];
-                o[8] = oacc[dm][e + 2];
+                to[16 * dm] = oacc[dm][e] * wt;
+                to[16 * dm + 8] = oacc[dm][e + 2] * wt;
+            }
+            if (c.g == 0) {
+                to[HD] = mm;
+                to[HD + 1] = l * wt;
             }
         }
     }
     res_sync();
     float* part = reinterpret_cast<float*>(ar + a.ar.part);
 #pragma unroll 1
-    for (uint32_t idx = threadIdx.x; idx < x.n_cols * HD; idx += RES_THREADS) {
-        const uint32_t p = idx / HD, d = idx % HD, pc = p / 8, cc = p % 8, tok = token_of(p);
-        float mm = -INFINITY, oo = 0.0f, ll = 0.0f;
-#pragma unroll 1
-        for (uint32_t w = pc; w < KG * NT; w += NT) mm = fmaxf(mm, sm.ml[w][0][cc]);
-        const float m0 = mm == -INFINITY ? 0.0f : mm;
-#pragma unroll 2
-        for (uint32_t w = pc; w < KG * NT; w += NT) {
-            const float wt = fast_exp2(sm.ml[w][0][cc] - m0);
-            ll += wt * sm.ml[w][1][cc];
-            oo += wt * red[(w * 8 + cc) * OS + d];
-        }
-        float* pp = part + (size_t((t0 + tok) * a.n_heads + x.kvh * a.heads_per_kv + p - tok * a.heads_per_kv) * a.max_splits + x.split) * ATTN_PART;
-        if (d == 0) {
-            st_word(pp, mm);
-            st_word(pp + 1, ll);
-        }
-        st_word(pp + 4 + d, oo);
+    for (uint32_t idx = threadIdx.x; idx < x.n_cols * OS; idx += RES_THREADS) {  // 64 sums, the maximum, l's sum (and two words of nothing)
+        const uint32_t p = idx / OS, d = idx % OS, tok = token_of(p);
+        const float* from = red + ((p / 8) * 8 + p % 8) * OS + d;
+        float sum = 0.0f;
+#pragma unroll 4
+        for (uint32_t w = 0; w < KG; w++) sum += from[w * NT * 8 * OS];
+        if (d == HD) sum = from[0];
+        if (d < HD + 2) st_word(part + (((t0 + tok) * a.n_heads + x.kvh * a.heads_per_kv + p - tok * a.heads_per_kv) * a.max_splits + x.split) * ATTN_PART + (d < HD ? 4 + d : d - HD), sum);
     }
     res_sync();  // (before the buffers' next use)
 }
 
-// The splits of every (token, head) merged: a block each, a warp a split at a time, two dims a lane.
+// The splits of every (token, head) merged: a block each, half a warp a split, four dims a lane.
 template <bool INT8>
 __device__ __forceinline__ void merge_phase(const DecodeArgs& a, DecodeSmem& sm, float* red, Ctx& c, uint32_t layer) {
     uint8_t* ar = layer_arena(a, layer);
 #pragma unroll 1
     for (uint32_t i = blockIdx.x; i < a.n * a.n_heads; i += gridDim.x) {
         uint32_t tok = 0;
+#pragma unroll 1
         for (uint32_t j = i; j >= a.n_heads; j -= a.n_heads) tok++;
         const uint32_t tile = sm.tok_tile[tok], S = a.unit0[tile + 1] - a.unit0[tile];
-        const float* pp = reinterpret_cast<const float*>(ar + a.ar.part) + size_t(i) * a.max_splits * ATTN_PART;
-        float m = -INFINITY, l = 0.0f, o0 = 0.0f, o1 = 0.0f;
-#pragma unroll 1
-        for (uint32_t s = c.warp; s < S; s += RES_WARPS) {
-            uint2 ml, o;
-            Patience p = patience(a, sm);
-            do {
-                ml = ld_word2(pp + s * ATTN_PART);
-                o = ld_word2(pp + s * ATTN_PART + 4 + 2 * c.lane);
-            } while (!(there(ml) && there(o)) && !p.over());
-            const float ms = __uint_as_float(ml.x), m_new = fmaxf(m, ms), m0 = m_new == -INFINITY ? 0.0f : m_new;
-            const float corr = exp2f(m - m0), w = exp2f(ms - m0);
+        const float* pp = reinterpret_cast<const float*>(ar + a.ar.part) + i * a.max_splits * ATTN_PART;
+        float m = -INFINITY, l = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        auto add = [&](float ms, float ls, const float (&x)[4]) {
+            const float m_new = fmaxf(m, ms), m0 = m_new == -INFINITY ? 0.0f : m_new;
+            const float corr = fast_exp2(m - m0), w = fast_exp2(ms - m0);
             m = m_new;
-            l = l * corr + w * __uint_as_float(ml.y);
-            o0 = o0 * corr + w * __uint_as_float(o.x);
-            o1 = o1 * corr + w * __uint_as_float(o.y);
+            l = l * corr + w * ls;
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[j] = o[j] * corr + w * x[j];
+        };
+#pragma unroll 1
+        for (uint32_t s0 = 0; s0 < S; s0 += 2 * RES_WARPS) {
+            const uint32_t s = s0 + 2 * c.warp + c.lane / 16;
+            uint2 ml = make_uint2(0xff800000u, 0u);
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (s < S) {
+                Patience p = patience(a, sm);
+                do {
+                    ml = ld_word2(pp + s * ATTN_PART);
+                    v = ld_word4(pp + s * ATTN_PART + 4 + 4 * (c.lane % 16));
+                } while (!(there(ml) && there(v)) && !p.over());
+            }
+            const float x[4] = {__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)};
+            add(__uint_as_float(ml.x), __uint_as_float(ml.y), x);
         }
         __syncwarp();
+        {  // the two halves, then the warps through shared memory
+            float x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = __shfl_xor_sync(0xffffffffu, o[j], 16);
+            add(__shfl_xor_sync(0xffffffffu, m, 16), __shfl_xor_sync(0xffffffffu, l, 16), x);
+        }
         res_sync();  // (the buffers' readers before are done)
-        float2* os = reinterpret_cast<float2*>(red) + c.warp * 33;
-        os[c.lane] = make_float2(o0, o1);
-        if (c.lane == 0) os[32] = make_float2(m, l);
+        float* to = red + c.warp * 68;
+        if (c.lane < 16) *reinterpret_cast<float4*>(to + 4 * c.lane) = make_float4(o[0], o[1], o[2], o[3]);
+        if (c.lane == 0) *reinterpret_cast<float2*>(to + 64) = make_float2(m, l);
         res_sync();
         if (c.warp == 0) {
-            const uint32_t live = min(S, RES_WARPS);
-            const float2* from = reinterpret_cast<const float2*>(red);
-            float mm = -INFINITY, ll = 0.0f, x0 = 0.0f, x1 = 0.0f;
-#pragma unroll 1
-            for (uint32_t w = 0; w < live; w++) mm = fmaxf(mm, from[w * 33 + 32].x);
-#pragma unroll 2
-            for (uint32_t w = 0; w < live; w++) {
-                const float2 ml = from[w * 33 + 32], o = from[w * 33 + c.lane];
-                const float wt = exp2f(ml.x - mm);
-                ll += wt * ml.y;
-                x0 += wt * o.x;
-                x1 += wt * o.y;
+            const float2 ml = c.lane < RES_WARPS ? *reinterpret_cast<const float2*>(red + c.lane * 68 + 64) : make_float2(-INFINITY, 0.0f);
+            const float w = fast_exp2(ml.x - warp_max(ml.x)), ll = warp_sum(w * ml.y);
+            float x0 = 0.0f, x1 = 0.0f;
+#pragma unroll 4
+            for (uint32_t j = 0; j < RES_WARPS; j++) {
+                const float2 v = *reinterpret_cast<const float2*>(red + j * 68 + 2 * c.lane);
+                const float wj = __shfl_sync(0xffffffffu, w, j);
+                x0 += wj * v.x;
+                x1 += wj * v.y;
             }
-            publish<INT8>(ar + a.ar.at, a.ar.half_o, size_t(i) * HD + 2 * c.lane, pack_bf16(x0 / ll, x1 / ll), scale_of(PH_O), 1, c.lane % 4 == 0);
+            publish<INT8>(ar + a.ar.at, a.ar.half_o, i * HD + 2 * c.lane, pack_bf16(x0 / ll, x1 / ll), scale_of(PH_O), 1, c.lane % 4 == 0);
         }
     }
 }
@@ -787,7 +816,8 @@ __global__ void __launch_bounds__(RES_THREADS + RES_ASKERS, 1) decode_kernel(con
         for (uint32_t at = blockIdx.x + i * gridDim.x; at < a.d / 16; at += 4 * gridDim.x, i += 4) {
             const float y = tok < a.n ? a.h[size_t(tok) * a.d + at * 16 + r] : 0.0f;
             sm.resid[i][tok][r] = y;
-            publish_resid<INT8>(a, a.arena, reinterpret_cast<float*>(a.arena + a.ar.ss1), at, tok, r, y);
+            tile_squares(a, reinterpret_cast<float*>(a.arena + a.ar.ss1), at, tok, r, y);
+            publish<INT8>(a.arena, a.ar.half_d, tok * a.d + at * 16 + r, pack_bf16(y, __shfl_down_sync(0xffffffffu, y, 1)), 1.0f, 2, tok < a.n && r % 8 == 0);
         }
     }
     res_sync();
@@ -886,6 +916,7 @@ void decode_split(DecodeArgs& a, const uint32_t* cached, uint32_t sm_count) {
         a.unit0[i + 1] = a.unit0[i] + s;
     }
     for (uint32_t i = nt + 1; i < 9; i++) a.unit0[i] = a.unit0[nt];
+    a.inv_d = 1.0f / float(a.d);
     a.n_units = a.unit0[nt] * nkv;
     a.heads_per_kv = a.n_heads / nkv;
     a.per_kv_recip = (65536 + a.heads_per_kv - 1) / a.heads_per_kv;

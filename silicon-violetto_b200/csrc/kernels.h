@@ -161,7 +161,7 @@ struct DecodeArgs {
     KvArgs kv;
     uint32_t split_pages, max_splits, unit0[9];  // of the cached keys: pages a split, the most splits of a tile, a tile's first split
     uint32_t n_units, heads_per_kv, per_kv_recip;  // units of the attention; query heads a kv head, and 65536 over that rounded up
-    float eps, scale_log2;
+    float eps, inv_d, scale_log2;
     const uint32_t *meta, *tiles, *vis, *page_table;
     const float* rope;
     uint16_t *k_cache, *v_cache;
