@@ -217,7 +217,7 @@ Engine::Engine(const std::string& weights, const EngineConfig& c, const Tuning& 
             lim->gates.alloc(n * md.n_heads * 4, false);
             lim->part.alloc(n * md.n_heads * size_t(LIMITE_MAX_SPLITS) * LIMITE_PART * 4, false);
         }
-        if (!model.limite) init_decode();
+        init_decode();
         VLT_CUDA(cudaDeviceSynchronize());
     }
 }
@@ -802,7 +802,7 @@ void Engine::init_decode() {
     int device_sms = 0, together = 0;
     VLT_CUDA(cudaDeviceGetAttribute(&device_sms, cudaDevAttrMultiProcessorCount, cfg.device));
     VLT_CUDA(cudaDeviceGetAttribute(&together, cudaDevAttrCooperativeLaunch, cfg.device));
-    if (!together || sm_count > uint32_t(device_sms) || !decode_fits(md, model.layers, sm_count)) return;
+    if (!together || sm_count > uint32_t(device_sms) || !decode_fits(md, model.limite, model.layers, sm_count)) return;
     std::vector<DecodeMap> maps;
     std::vector<const uint16_t*> scales;
     auto put = [&](const Matrix& m) {
@@ -812,14 +812,14 @@ void Engine::init_decode() {
     };
     for (const Layer& l : model.layers)
         for (const Matrix* m : {&l.qkv, &l.o, &l.gate_up, &l.down}) put(*m);
-    if (decode_head_fits()) put(model.head);
+    if (!model.limite && decode_head_fits()) put(model.head);
     dec.maps.alloc(maps.size() * sizeof(DecodeMap), false);
     dec.maps.write_vec(0, maps);
     dec.scales.alloc(scales.size() * sizeof(scales[0]), false);
     dec.scales.write_vec(0, scales);
     dec.most = std::min(8u, cfg.max_step_tokens);
-    const DecodeArena a = decode_arena(md, model.layers[0].qkv.int8, dec.most, decode_max_splits(md.n_kv, sm_count));
-    for (Buffer& b : dec.words) b.alloc(size_t(md.n_layers) * a.layer_bytes + a.q, false);
+    const DecodeArena a = decode_arena(md, model.layers[0].qkv.int8, dec.most, model.limite ? 0u : decode_max_splits(md.n_kv, sm_count));
+    for (Buffer& b : dec.words) b.alloc(size_t(model.limite ? 1 : md.n_layers) * a.layer_bytes + a.q, false);
     reset_decode();
 }
 
@@ -836,22 +836,46 @@ bool Engine::use_decode(const Plan& p) const {
     return p.n <= dec.most && p.tiles == p.n_runs && p.tiles * model.md.n_kv <= DECODE_UNITS * sm_count && !p.chunked && !skip && !profile && !tuning.plain_attention && !tuning.attn_keys_per_cta && !tuning.gemm_min_rows;
 }
 
-void Engine::encode_decode(uint32_t set, const Plan& p) {
-    StepSet& st = sets[set];
+DecodeArgs Engine::decode_args(uint32_t n) const {
     const ModelDesc& md = model.md;
-    const Layer& first = model.layers[0];
     DecodeArgs a{};
     a.maps = dec.maps.as<DecodeMap>();
     a.scales = dec.scales.as<const uint16_t*>();
     a.n_layers = md.n_layers;
-    a.n = p.n;
-    a.n_tiles = p.tiles;
+    a.n = n;
     a.d = md.d;
     a.ffn = md.ffn;
     a.n_heads = md.n_heads;
+    a.attn_w = md.n_heads * md.hd;
+    a.qkv_w = md.qkv_w();
+    a.eps = md.eps;
+    a.inv_d = 1.0f / float(md.d);
+    a.err_flag = s.err_flag.as<uint32_t>();
+    return a;
+}
+
+void Engine::run_decode(DecodeArgs& a, uint32_t s0, uint32_t s1) {
+    const uint32_t turn = dec.turn, other = turn ^ 1u;
+    a.s0 = s0;
+    a.s1 = s1;
+    a.l0 = s0 / 5;
+    a.l1 = s1 / 5;
+    a.arena = dec.words[turn].as<uint8_t>();
+    a.clear = dec.words[other].as<uint8_t>();
+    a.clear_bytes = dec.used[other];
+    launch_decode(a, attn_maps, model.layers[0].qkv.int8, sm_count, stream);
+    dec.used[turn] = size_t(a.l1 - a.l0) * a.ar.layer_bytes + a.ar.q;  // (what a layer's down leaves lies where the next one's words begin)
+    dec.used[other] = 0;
+    dec.turn = other;
+}
+
+void Engine::encode_decode(uint32_t set, const Plan& p) {
+    StepSet& st = sets[set];
+    const ModelDesc& md = model.md;
+    DecodeArgs a = decode_args(p.n);
+    a.n_tiles = p.tiles;
     a.kv = kv_args();
     decode_split(a, p.cached, sm_count);
-    a.eps = md.eps;
     a.scale_log2 = md.attn_scale * 1.44269504088896340736f;
     a.meta = s.meta.as<uint32_t>();
     a.tiles = st.in<uint32_t>(st.o_tiles);
@@ -861,15 +885,13 @@ void Engine::encode_decode(uint32_t set, const Plan& p) {
     a.k_cache = kv.k.as<uint16_t>();
     a.v_cache = kv.v.as<uint16_t>();
     a.h = s.h.as<float>();
-    a.ar = decode_arena(md, first.qkv.int8, p.n, a.max_splits);
-    a.err_flag = s.err_flag.as<uint32_t>();
+    a.out = s.h.as<float>();
+    a.ar = decode_arena(md, model.layers[0].qkv.int8, p.n, a.max_splits);
     // A launch ends behind each tapped layer: the tap is a row pass over its output.
     for (uint32_t l0 = 0, l1; l0 < md.n_layers; l0 = l1) {
         l1 = md.n_layers;
         for (uint32_t t : tap_layers)
             if (t >= l0 && t + 1 < l1) l1 = t + 1;
-        a.l0 = l0;
-        a.l1 = l1;
         if (l1 == md.n_layers && decode_head(p)) {
             a.head_s = model.head.scales;
             a.head_rows = st.in<uint32_t>(st.o_head_rows);
@@ -878,14 +900,7 @@ void Engine::encode_decode(uint32_t set, const Plan& p) {
             a.vocab = md.vocab;
             a.vocab_real = md.vocab_real;
         }
-        const uint32_t turn = dec.turn, other = turn ^ 1u;
-        a.arena = dec.words[turn].as<uint8_t>();
-        a.clear = dec.words[other].as<uint8_t>();
-        a.clear_bytes = dec.used[other];
-        launch_decode(a, attn_maps, first.qkv.int8, sm_count, stream);
-        dec.used[turn] = size_t(l1 - l0) * a.ar.layer_bytes + a.ar.q;
-        dec.used[other] = 0;
-        dec.turn = other;
+        run_decode(a, 5 * l0, 5 * l1);
         auto tap = std::find(tap_layers.begin(), tap_layers.end(), l1 - 1);
         if (tap != tap_layers.end())
             launch_prep_rows(s.h.as<float>(), nullptr, p.n, md.d, md.eps, tap_bufs[tap - tap_layers.begin()].as<float>(), nullptr, nullptr, true, true, stream);
@@ -930,6 +945,16 @@ void Engine::encode_forward_limite(uint32_t set, const Plan& p) {
         return gemm_fits(l.qkv, n) && gemm_fits(l.o, n) && gemm_fits(l.gate_up, n) && gemm_fits(l.down, n) && md.n_heads / md.n_kv <= 8 && md.d % 128 == 0;
     };
     auto mudd_site = [](uint32_t li) { return li == 24 ? 0 : li == 47 ? 1 : -1; };  // model.rs:20 `MUDD_LAYERS`
+    // Steps of at most 8 tokens: a layer's o, gate_up and down, and the next layer's qkv unless a MUDD mix comes in between, in one
+    // launch (k_decode.cu), where each was one: 8 streams over 2 048 keys took 2 237 us a step.
+    const bool fused = n <= dec.most && !profile && !tuning.gemm_min_rows && md.n_heads / md.n_kv <= 8;
+    DecodeArgs da = decode_args(n);
+    if (fused) {
+        da.attn = s.attn_b.as<uint8_t>();
+        da.qkv = s.qkv.as<float>();
+        da.inv_out = s.inv.as<float>();
+        da.ar = decode_arena(md, false, n, 0);
+    }
     for (uint32_t li = 0; li < md.n_layers; li++) {
         const Layer& l = model.layers[li];
         const LimiteLayer& x = model.lim[li];
@@ -956,6 +981,12 @@ void Engine::encode_forward_limite(uint32_t set, const Plan& p) {
         if (big) {
             if (!carried) launch_prep_rows(xa, nullptr, n, H, md.eps, nullptr, s.h_b.as<uint16_t>(), s.inv.as<float>(), false, false, stream);
             matmul_gemm(l.qkv, n, s.h_b.as<uint16_t>(), s.qkv.as<float>(), nullptr, EPI_NORM, nullptr, inv_in, 0, nullptr, nullptr, ssq_in, x.qkv_scale);
+        } else if (fused) {
+            if (li == 0 || site >= 0) {
+                da.h = xa;
+                da.lim.qkv_scale = x.qkv_scale;
+                run_decode(da, 5 * li, 5 * li + 1);
+            }
         } else {
             matmul(l.qkv, n, xa, s.qkv.as<float>(), EPI_NORM, nullptr, s.inv.as<float>(), 0, nullptr, nullptr, nullptr, x.qkv_scale);
         }
@@ -966,7 +997,7 @@ void Engine::encode_forward_limite(uint32_t set, const Plan& p) {
         span_end(sp);
         sp = span_begin(G_ATTN);
         launch_limite_attn(s.qkv.as<float>(), meta, tin, st.in<uint32_t>(st.o_vis), st.in<uint32_t>(st.o_tiles), p.tiles, kc, vc, kva, md.n_heads, LIMITE_WINDOW, md.attn_scale, L.vdir.as<float>(), L.gates.as<float>(), x.xsa,
-                           n, (x.global ? p.max_keys : std::min(p.max_keys, LIMITE_WINDOW)) + 8, L.part.as<float>(), s.attn.as<float>(), big ? s.attn_b.as<uint16_t>() : nullptr, tuning.attn_keys_per_cta, stream);
+                           n, (x.global ? p.max_keys : std::min(p.max_keys, LIMITE_WINDOW)) + 8, L.part.as<float>(), s.attn.as<float>(), big || fused ? s.attn_b.as<uint16_t>() : nullptr, tuning.attn_keys_per_cta, stream);
         span_end(sp);
         sp = span_begin(G_MATMUL);
         float* out = li == 11 ? L.hist12.as<float>() : li == 22 ? L.hist23.as<float>() : s.h.as<float>();  // encode.rs:116-122 `resid_out`
@@ -977,6 +1008,12 @@ void Engine::encode_forward_limite(uint32_t set, const Plan& p) {
             const bool carry = li + 1 < md.n_layers && big_of(li + 1) && mudd_site(li + 1) < 0;
             matmul_gemm(l.down, n, s.act_b.as<uint16_t>(), out, carry ? s.h_b.as<uint16_t>() : nullptr, EPI_RESID, L.mixed.as<float>(), nullptr, 0, nullptr,
                         carry ? s.ssq.as<float>() : nullptr, nullptr, 1.0f, x.resid_mlp, x.post_mlp);
+        } else if (fused) {
+            const bool on = li + 1 < md.n_layers && mudd_site(li + 1) < 0;
+            da.h = base;
+            da.out = out;
+            da.lim = {on ? model.lim[li + 1].qkv_scale : 0.0f, x.o_scale, x.resid_attn, x.post_attn, x.resid_mlp, x.post_mlp};
+            run_decode(da, 5 * li + 2, 5 * (li + 1) + (on ? 1 : 0));
         } else {
             matmul(l.o, n, s.attn.as<float>(), L.mixed.as<float>(), EPI_RESID, base, nullptr, 0, nullptr, nullptr, nullptr, x.o_scale, x.resid_attn, x.post_attn);
             matmul(l.gate_up, n, L.mixed.as<float>(), s.act.as<float>(), EPI_SWIGLU, nullptr, nullptr);

@@ -240,6 +240,8 @@ class Engine {
     bool decode_head_fits() const;
     bool decode_head(const Plan& p) const;
     void encode_decode(uint32_t set, const Plan& p);
+    DecodeArgs decode_args(uint32_t n) const;
+    void run_decode(DecodeArgs& a, uint32_t s0, uint32_t s1);  // one launch on the next set of words
     // The chain drafter (a benchmark extension; the reference's drafter.rs is a block drafter): fc over
     // (feature ; embedding), one decoder layer with a cache of its own on the target's page table, a head
     // over a draft vocabulary.

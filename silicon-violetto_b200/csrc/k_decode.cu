@@ -60,9 +60,9 @@ struct DecodeSmem {
 // A block's first row tile; it takes every gridDim.x-th from there. qkv counts from the other end, so that the blocks without a
 // tile of o and down have the second ones of qkv.
 __device__ __forceinline__ uint32_t first_tile(uint32_t ph) { return ph == PH_QKV ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }
-__device__ __forceinline__ uint32_t width_of(const DecodeArgs& a, uint32_t ph) { return ph == PH_O ? a.n_heads * HD : ph == PH_DOWN ? a.ffn : a.d; }
+__device__ __forceinline__ uint32_t width_of(const DecodeArgs& a, uint32_t ph) { return ph == PH_O ? a.attn_w : ph == PH_DOWN ? a.ffn : a.d; }
 __device__ __forceinline__ uint32_t tiles_of(const DecodeArgs& a, uint32_t ph) {
-    return (ph == PH_HEAD ? a.vocab : ph == PH_QKV ? (a.n_heads + 2 * a.kv.n_kv) * HD : ph == PH_GU ? 2 * a.ffn : a.d) / 16;
+    return (ph == PH_HEAD ? a.vocab : ph == PH_QKV ? a.qkv_w : ph == PH_GU ? 2 * a.ffn : a.d) / 16;
 }
 
 __device__ __forceinline__ Unit unit_of(const DecodeArgs& a, const DecodeSmem& sm, uint32_t u) {
@@ -101,26 +101,25 @@ __device__ __forceinline__ void ask(const DecodeArgs& a, const AttnMaps& maps, D
         if (lane == 0) *const_cast<volatile uint32_t*>(&sm.asked) = item;
         return st;
     };
-    // Lanes 0 .. 3: the layer's scales, fetched while the layer before is asked for (the head's in lane 0, behind the last layer).
-    const uint16_t* coming = nullptr;
-    uint32_t matrix = 4 * a.l0;  // the layer's first
+    // Lanes 0 .. 3: the layer's scales, fetched while the layer before is asked for (behind the last layer the head's, in lane 0).
+    auto fetch = [&](uint32_t layer) -> const uint16_t* {
+        const uint32_t i = layer < a.n_layers ? 4 * layer + lane : 4 * a.n_layers;
+        if (lane >= (layer < a.n_layers ? 4u : a.n_head ? 1u : 0u)) return nullptr;
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&a.maps[i]) : "memory");
+        return a.wbytes == 1 ? a.scales[i] : nullptr;
+    };
+    const uint16_t *at_hand = nullptr, *coming = fetch(a.s0 / PH_HEAD);
+    uint32_t layer = a.s0 / PH_HEAD, ph = a.s0 % PH_HEAD;
+    bool turned = true;
 #pragma unroll 1
-    for (uint32_t ahead = 0;; ahead = 1, matrix += 4) {
-        const uint16_t* at_hand = coming;
-        if (matrix == 4 * a.l1 + (a.n_head ? 4u : 0u)) break;
-        const bool last = matrix + 4 * ahead >= 4 * a.l1;  // (the first time round the layer itself is fetched)
-        const uint32_t next = last ? 4 * a.n_layers : matrix + 4 * ahead + lane;
-        if (lane < (last ? a.n_head != 0 : 4)) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&a.maps[next]) : "memory");
-            if (a.wbytes == 1) coming = a.scales[next];
+    for (uint32_t s = a.s0; s < a.s1 + (a.n_head ? 1u : 0u); s++) {
+        if (turned) {
+            at_hand = coming;
+            coming = fetch(layer + 1);
+            turned = false;
         }
-        if (!ahead) {
-            matrix -= 4;
-            continue;
-        }
-        const bool head = matrix == 4 * a.l1;
-#pragma unroll 1
-        for (uint32_t ph = head ? PH_HEAD : PH_QKV; ph < (head ? PH_END : PH_HEAD); ph++) {
+        if (s == a.s1) ph = PH_HEAD;
+        {
             if (ph == PH_ATTN) {
                 uint32_t listed = 0;
 #pragma unroll 1
@@ -133,15 +132,17 @@ __device__ __forceinline__ void ask(const DecodeArgs& a, const AttnMaps& maps, D
                         __syncwarp();
                         if (lane < count) {
                             const uint32_t id = listed + lane < LISTED ? sm.ids[listed + lane] : a.page_table[size_t(sm.slot[x.tile]) * a.kv.max_pages + x.page0 + first + lane];
-                            const int y = int(((matrix / 4 * a.kv.n_pages + id) * a.kv.n_kv + x.kvh) * PAGE);
+                            const int y = int(((layer * a.kv.n_pages + id) * a.kv.n_kv + x.kvh) * PAGE);
                             const uint32_t to = stages + st * RES_STAGE + lane * PAGE_BYTES;
                             tile_load(to, &maps.k, 0, y, bar);
                             tile_load(to + PAGE_BYTES / 2, &maps.v, 0, y, bar);
                         }
                     }
                 }
+                ph++;
                 continue;
             }
+            const bool head = ph == PH_HEAD;
             const uint32_t which = ph == PH_QKV || head ? 0u : ph - 1;
             const uint16_t* scales = reinterpret_cast<const uint16_t*>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(at_hand), which));
 #pragma unroll 1
@@ -152,11 +153,16 @@ __device__ __forceinline__ void ask(const DecodeArgs& a, const AttnMaps& maps, D
                     const bool with = a.wbytes == 1 && (part + 1) * RES_SLICE >= width_of(a, ph);
                     if (lane == 0) {
                         bar_expect(bar, RES_ITEM + (with ? 32u : 0u));  // (what a box has beyond the matrix counts, and is zero)
-                        tile_load(dst, &a.maps[head ? 4 * a.n_layers : matrix + which], 0, int(at * 16), int(part * 16), bar);
+                        tile_load(dst, &a.maps[head ? 4 * a.n_layers : 4 * layer + which], 0, int(at * 16), int(part * 16), bar);
                         if (with) bulk_load(dst + RES_ITEM, scales + at * 16, 32, bar);
                     }
                     __syncwarp();
                 }
+            if (++ph == PH_HEAD) {
+                ph = PH_QKV;
+                layer++;
+                turned = true;
+            }
         }
     }
 }
@@ -262,7 +268,7 @@ struct Squares {
 
 // One matmul phase: the block's row tiles of a matrix against the activations x [token][k] (bf16, polled for), the epilogue by phase.
 // Columns past the tokens repeat the last one's (nothing reads their sums).
-template <bool INT8>
+template <bool INT8, bool LIMITE>
 __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm, uint8_t* stages, float* red, uint4* xs, Ctx& c, uint32_t layer, uint32_t ph, const uint8_t* words, const float* ss) {
     using P = Piece<INT8>;
     constexpr uint32_t WB = P::WB, E = P::E, R = P::R, KS = E / 4, PARTS = INT8 ? 1 : 2, CHUNK = 2;  // a group's parts of a row; pieces whose operands a warp holds (at most 32 registers)
@@ -441,6 +447,11 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
         if (ph == PH_HEAD) {
             const uint32_t at = tile * 16 + r;
             if (tok < a.n_head) a.logits[size_t(tok) * a.vocab + at] = at < a.vocab_real ? sum : -INFINITY;
+        } else if (LIMITE && ph == PH_QKV) {  // (the rest of this architecture's qkv work is a kernel of its own)
+            if (tok < a.n) {
+                a.qkv[tok * a.qkv_w + tile * 16 + r] = sum * a.lim.qkv_scale;
+                if (tile == 0 && r == 0) a.inv_out[tok] = inv;
+            }
         } else if (ph == PH_QKV) {
             // RoPE on q and k; q scaled for the attention; k and v into the cache and, for this step's attention, beside it.
             const uint32_t head = tile / (HD / 16), pair = (tile % (HD / 16)) * 8 + r / 2;
@@ -471,13 +482,14 @@ __device__ __forceinline__ void matmul_phase(const DecodeArgs& a, DecodeSmem& sm
                 at = tok * a.ffn + tile * 8 + r / 2;
             } else {
                 float& h = sm.resid[i_tile][tok][r];
-                h += sum;
+                if (LIMITE) h = ph == PH_O ? a.lim.ra * h + a.lim.rb * (a.lim.o_scale * sum) : a.lim.ra2 * h + a.lim.rb2 * sum;
+                else h += sum;
                 y = h;
                 to = ph == PH_O ? a.ar.x2 : a.ar.layer_bytes;  // (what down leaves is the next layer's input, or the head's)
                 at = tok * a.d + tile * 16 + r;
-                if (ph == PH_DOWN && layer + 1 == a.l1) {
-                    if (tok < a.n) a.h[at] = y;
-                    if (!a.n_head) continue;
+                if (ph == PH_DOWN && (LIMITE || layer + 1 == a.l1)) {
+                    if (tok < a.n) a.out[at] = y;
+                    if (layer * PH_HEAD + PH_DOWN + 1 == a.s1 && !a.n_head) continue;  // (nothing follows in this launch)
                 }
                 tile_squares(a, reinterpret_cast<float*>(ar + to + (ph == PH_O ? a.ar.ss2 - a.ar.x2 : a.ar.ss1)), tile, tok, r, y);
             }
@@ -738,7 +750,9 @@ __device__ __forceinline__ void merge_phase(const DecodeArgs& a, DecodeSmem& sm,
     }
 }
 
-template <bool INT8>
+// LIMITE: the reference's own architecture, whose attention has kernels of its own: a launch is a qkv phase, or o, gate_up, down and,
+// where nothing comes in between, the next layer's qkv; scales and residual lambdas as MatArgs has them.
+template <bool INT8, bool LIMITE>
 __global__ void __launch_bounds__(RES_THREADS + RES_ASKERS, 1) decode_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ AttnMaps maps) {
     extern __shared__ uint8_t decode_smem_raw[];
     uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(decode_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -798,7 +812,7 @@ __global__ void __launch_bounds__(RES_THREADS + RES_ASKERS, 1) decode_kernel(con
     c.t = c.lane & 3;
     c.items = 0;
     c.turn = 0;
-    if (tid < 256) {
+    if (!LIMITE && tid < 256) {
         const uint32_t tok = tid / 32, pair = tid % 32;
         if (tok < a.n) {
             sm.cs[tok][pair] = reinterpret_cast<const float2*>(a.rope)[size_t(a.meta[2 * tok + 1]) * (HD / 2) + pair];
@@ -816,28 +830,31 @@ __global__ void __launch_bounds__(RES_THREADS + RES_ASKERS, 1) decode_kernel(con
         for (uint32_t at = blockIdx.x + i * gridDim.x; at < a.d / 16; at += 4 * gridDim.x, i += 4) {
             const float y = tok < a.n ? a.h[size_t(tok) * a.d + at * 16 + r] : 0.0f;
             sm.resid[i][tok][r] = y;
+            if (LIMITE && a.s0 % PH_HEAD != PH_QKV) continue;
             tile_squares(a, reinterpret_cast<float*>(a.arena + a.ar.ss1), at, tok, r, y);
             publish<INT8>(a.arena, a.ar.half_d, tok * a.d + at * 16 + r, pack_bf16(y, __shfl_down_sync(0xffffffffu, y, 1)), 1.0f, 2, tok < a.n && r % 8 == 0);
         }
     }
     res_sync();
+    uint32_t layer = a.s0 / PH_HEAD, ph = a.s0 % PH_HEAD;
 #pragma unroll 1
-    for (uint32_t layer = a.l0; layer < a.l1 + (a.n_head ? 1u : 0u); layer++) {
-        const uint8_t* ar = layer_arena(a, layer);
-        const bool head = layer == a.l1;
+    for (uint32_t s = a.s0; s < a.s1 + (a.n_head ? 1u : 0u); s++) {
+        if (s == a.s1) ph = PH_HEAD;
+        c.renew();
+        if (!LIMITE && ph == PH_ATTN) {
 #pragma unroll 1
-        for (uint32_t ph = head ? PH_HEAD : PH_QKV; ph < (head ? PH_END : PH_HEAD); ph++) {
+            for (uint32_t u = 0; u * gridDim.x + blockIdx.x < a.n_units; u++) attention_unit(a, sm, stages, red, xs, c, layer, sm.unit[u]);
             c.renew();
-            if (ph == PH_ATTN) {
-#pragma unroll 1
-                for (uint32_t u = 0; u * gridDim.x + blockIdx.x < a.n_units; u++) attention_unit(a, sm, stages, red, xs, c, layer, sm.unit[u]);
-                c.renew();
-                merge_phase<INT8>(a, sm, red, c, layer);
-                continue;
-            }
-            const uint32_t x_off = ph == PH_O ? a.ar.at : ph == PH_GU ? a.ar.x2 : ph == PH_DOWN ? a.ar.act : 0u;
+            merge_phase<INT8>(a, sm, red, c, layer);
+        } else {
+            const uint8_t* ar = layer_arena(a, layer);
+            const uint8_t* x = LIMITE && ph == PH_O ? a.attn : ar + (ph == PH_O ? a.ar.at : ph == PH_GU ? a.ar.x2 : ph == PH_DOWN ? a.ar.act : 0u);
             const uint8_t* ss = ph == PH_QKV || ph == PH_HEAD ? ar + a.ar.ss1 : ph == PH_GU ? ar + a.ar.ss2 : nullptr;
-            matmul_phase<INT8>(a, sm, stages, red, xs, c, layer, ph, ar + x_off, reinterpret_cast<const float*>(ss));
+            matmul_phase<INT8, LIMITE>(a, sm, stages, red, xs, c, layer, ph, x, reinterpret_cast<const float*>(ss));
+        }
+        if (++ph == PH_HEAD) {
+            ph = PH_QKV;
+            layer++;
         }
     }
 }
@@ -846,12 +863,13 @@ __global__ void __launch_bounds__(RES_THREADS + RES_ASKERS, 1) decode_kernel(con
 constexpr size_t DECODE_SMEM = size_t(RES_STAGES) * RES_STAGE + RES_RED * 4 + RES_X + 1024;
 static_assert(DECODE_SMEM + sizeof(DecodeSmem) + 256 <= 227 * 1024, "a block's shared memory");
 
-bool decode_fits(const ModelDesc& md, const std::vector<Layer>& layers, uint32_t sm_count) {
-    if (md.hd != HD || md.page != PAGE || md.n_heads % md.n_kv || md.n_heads / md.n_kv > 4 || layers.empty()) return false;
+bool decode_fits(const ModelDesc& md, bool limite, const std::vector<Layer>& layers, uint32_t sm_count) {
+    if (layers.empty() || (!limite && (md.hd != HD || md.page != PAGE || md.n_heads % md.n_kv || md.n_heads / md.n_kv > 4))) return false;
     const bool int8 = layers[0].qkv.int8;
-    const uint32_t wb = int8 ? 1 : 2, most = 8192;  // (a team is at most four groups, a group's parts 2 KiB of int8 and 4 of bf16)
-    if (md.d > most || md.ffn > most || md.n_heads * HD > most) return false;
-    if (md.d % 256 || md.ffn % 256 || (md.n_heads * HD) % 256 || md.n_heads * HD * wb % RES_PIECE) return false;
+    const uint32_t wb = int8 ? 1 : 2, most = 8192, attn_w = md.n_heads * md.hd;  // (a team is at most four groups, a group's parts 2 KiB of int8 and 4 of bf16)
+    if (limite && int8) return false;  // (its attention leaves no fp16 words)
+    if (md.d > most || md.ffn > most || attn_w > most) return false;
+    if (md.d * wb % RES_PIECE || md.ffn * wb % RES_PIECE || attn_w * wb % RES_PIECE || md.d % 16 || md.ffn % 8 || md.qkv_w() % 16) return false;
     if ((md.d / 16 + sm_count - 1) / sm_count > DECODE_RESID_TILES) return false;
     for (const Layer& l : layers)
         for (const Matrix* m : {&l.qkv, &l.o, &l.gate_up, &l.down}) {
@@ -916,7 +934,6 @@ void decode_split(DecodeArgs& a, const uint32_t* cached, uint32_t sm_count) {
         a.unit0[i + 1] = a.unit0[i] + s;
     }
     for (uint32_t i = nt + 1; i < 9; i++) a.unit0[i] = a.unit0[nt];
-    a.inv_d = 1.0f / float(a.d);
     a.n_units = a.unit0[nt] * nkv;
     a.heads_per_kv = a.n_heads / nkv;
     a.per_kv_recip = (65536 + a.heads_per_kv - 1) / a.heads_per_kv;
@@ -928,8 +945,9 @@ void launch_decode(DecodeArgs a, const AttnMaps& maps, bool int8, uint32_t sm_co
     a.wbytes = int8 ? 1 : 2;
     static PerDevice configured;
     configured.once([] {
-        VLT_CUDA(cudaFuncSetAttribute(decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DECODE_SMEM)));
-        VLT_CUDA(cudaFuncSetAttribute(decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DECODE_SMEM)));
+        VLT_CUDA(cudaFuncSetAttribute(decode_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DECODE_SMEM)));
+        VLT_CUDA(cudaFuncSetAttribute(decode_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DECODE_SMEM)));
+        VLT_CUDA(cudaFuncSetAttribute(decode_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(DECODE_SMEM)));
     });
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count);
@@ -941,8 +959,9 @@ void launch_decode(DecodeArgs a, const AttnMaps& maps, bool int8, uint32_t sm_co
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (int8) VLT_CUDA(cudaLaunchKernelEx(&cfg, decode_kernel<true>, a, maps));
-    else VLT_CUDA(cudaLaunchKernelEx(&cfg, decode_kernel<false>, a, maps));
+    if (a.attn) VLT_CUDA(cudaLaunchKernelEx(&cfg, decode_kernel<false, true>, a, maps));
+    else if (int8) VLT_CUDA(cudaLaunchKernelEx(&cfg, decode_kernel<true, false>, a, maps));
+    else VLT_CUDA(cudaLaunchKernelEx(&cfg, decode_kernel<false, false>, a, maps));
     launch_counter().fetch_add(1, std::memory_order_relaxed);
 }
 

@@ -156,8 +156,9 @@ struct DecodeArena {                          // where a layer's words lie (x1, 
 struct DecodeArgs {
     const DecodeMap* maps;                    // [layer][qkv, o, gate_up, down], then the head's
     const uint16_t* const* scales;            // the same (NULL: bf16)
+    uint32_t s0, s1;                          // phases from s0 on, up to s1: 5 layer + (0 qkv, 1 attention, 2 o, 3 gate_up, 4 down)
     uint32_t n_layers, l0, l1, n, n_tiles;              // tokens; attention tiles, one a run
-    uint32_t d, ffn, n_heads;
+    uint32_t d, ffn, n_heads, attn_w, qkv_w;  // attn_w, qkv_w: columns of o, rows of qkv
     KvArgs kv;
     uint32_t split_pages, max_splits, unit0[9];  // of the cached keys: pages a split, the most splits of a tile, a tile's first split
     uint32_t n_units, heads_per_kv, per_kv_recip;  // units of the attention; query heads a kv head, and 65536 over that rounded up
@@ -165,7 +166,12 @@ struct DecodeArgs {
     const uint32_t *meta, *tiles, *vis, *page_table;
     const float* rope;
     uint16_t *k_cache, *v_cache;
-    float* h;                                 // [n][d], in and out
+    const float* h;                           // [n][d], the residual stream that comes in
+    float* out;                               // and the one that goes out
+    // The reference's own architecture (attn: its attention's rows in bf16; NULL: a plain decoder).
+    const uint8_t* attn;
+    float *qkv, *inv_out;                     // [n][qkv_w], normed and scaled; [n] 1 / rms of what came in
+    struct { float qkv_scale, o_scale, ra, rb, ra2, rb2; } lim;
     uint8_t *arena, *clear;                   // this launch's words (all ones), and the other set, to be made so
     size_t clear_bytes;
     DecodeArena ar;
@@ -176,7 +182,7 @@ struct DecodeArgs {
     uint32_t wbytes;                          // (launch_decode's)
     uint32_t* err_flag;
 };
-bool decode_fits(const ModelDesc& md, const std::vector<Layer>& layers, uint32_t sm_count);
+bool decode_fits(const ModelDesc& md, bool limite, const std::vector<Layer>& layers, uint32_t sm_count);
 inline uint32_t decode_max_splits(uint32_t n_kv, uint32_t sm_count) { return sm_count > n_kv ? sm_count / n_kv : 1u; }
 DecodeArena decode_arena(const ModelDesc& md, bool int8, uint32_t n, uint32_t max_splits);
 void decode_split(DecodeArgs& a, const uint32_t* cached, uint32_t sm_count);  // cached: each tile's keys before the step, at most

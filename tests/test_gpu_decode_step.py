@@ -4,7 +4,7 @@ stage, of several, of a part that is not whole, groups of warps that share a row
 units to a block, contexts around the edges of pages and splits -- and over activations that fp16 does not hold as they are.
 
 Both multiply the same bf16 activations; sums are in another order, and through it a rounding to bf16 (2^-9) falls otherwise now
-and then: over two layers the results may differ by a few such roundings' share, 1e-2 in the 2-norm.
+and then: over two layers the results may differ by a few such roundings' share, 1e-2 in the 2-norm; over 26 layers by 3e-2.
 """
 import numpy as np
 import pytest
@@ -68,22 +68,22 @@ def _near(got, want, bound=1e-2):
     assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want)
 
 
-def _compare(engines, runs, launches=None, **opts):
+def _compare(engines, runs, launches=None, bound=1e-2, caches=("k_cache", "v_cache"), **opts):
     opts = E.StepOptions(head=E.Rows.ALL, hidden=E.Rows.ALL, read_logits=True, **opts)
-    outs, caches = [], []
+    outs, kept = [], []
     for i, eng in enumerate(engines):
         seqs = [_context(eng, n, 10 + j) for j, (n, _) in enumerate(runs)]
         before = eng.launches()
         outs.append(eng.step([E.Run(s, _ids(k, 50 + j)) for j, (s, (_, k)) in enumerate(zip(seqs, runs))], opts))
         if launches is not None and i == 0:
             assert eng.launches() - before <= launches  # (embedding, the layers and the head, hidden rows, sampling, acceptance)
-        caches.append([vlt.from_bf16(eng.debug_read(c).view(np.uint16)) for c in ("k_cache", "v_cache")])
+        kept.append([vlt.from_bf16(eng.debug_read(c).view(np.uint16)) for c in caches])
         for s in seqs:
             eng.free_seq(s)
-    _near(outs[0].logits, outs[1].logits)
-    _near(outs[0].hidden, outs[1].hidden)
-    for a, b in zip(*caches):
-        _near(a, b)
+    _near(outs[0].logits, outs[1].logits, bound)
+    _near(outs[0].hidden, outs[1].hidden, bound)
+    for a, b in zip(*kept):
+        _near(a, b, bound)
     return outs
 
 
@@ -123,3 +123,14 @@ def test_taps_between_launches(weights):
         eng.set_taps([0, 1])
     a, b = _compare(engines, RUNS["mixed"], read_taps=True)
     _near(vlt.from_bf16(np.asarray(a.taps, np.uint16)), vlt.from_bf16(np.asarray(b.taps, np.uint16)))
+
+
+# The reference's own architecture: o, gate_up, down and the next layer's qkv in one launch, up to a MUDD mix (in front of layers 24
+# and 47) -- rows of 768 bytes (a stage half full), of a stage and a quarter, and feed-forwards of two parts and a bit.
+@pytest.mark.parametrize("hidden,ffn", [(384, 640), (1280, 2112)])
+@pytest.mark.parametrize("runs", ["one", "drafts", "mixed", "eight"])
+def test_the_reference_architecture(tmp_path, hidden, ffn, runs):
+    path = tmp_path / "w.vlt"
+    synth.write_limite(path, n_layers=26, hidden=hidden, n_kv=1 if hidden == 384 else 2, ffn=ffn, vocab=512, seed=5)
+    cfg = dict(max_seqs=8, max_step_tokens=256, max_chunk=256, global_kv_tokens=8 * 1024, max_seq_len=1024, max_head_rows=8)
+    _compare([E.Engine(path, E.EngineConfig(**cfg), E.Tuning(gemm_min_rows=m)) for m in (0, 9)], RUNS[runs], launches=4 * 26 + 12, bound=3e-2, caches=())
