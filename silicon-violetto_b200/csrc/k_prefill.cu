@@ -178,18 +178,34 @@ __global__ void __launch_bounds__(GROUPS * WARPS * 32, blocks_per_sm(GROUPS)) at
                         if (!seen) sacc[j][e] = -INFINITY;
                     }
             }
-            // Online softmax: a row's 64 scores sit in the four lanes of its quad.
-            float corr[2];
+            // Online softmax, a row's 64 scores in the four lanes of its quad, with a lazy maximum as in the decode kernel
+            // (k_attn.cu): it only has to keep 2^(s - m) in range, so it moves, and the sums so far are rescaled, when a score of
+            // the block exceeds it by more than 8 -- one vote in place of the quads' reductions and 32 products a thread.
+            float mx[2];
 #pragma unroll
             for (int r = 0; r < 2; r++) {
-                float mx = -INFINITY;
+                mx[r] = -INFINITY;
 #pragma unroll
-                for (int j = 0; j < 8; j++) mx = fmaxf(mx, fmaxf(sacc[j][2 * r], sacc[j][2 * r + 1]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float m_new = fmaxf(m_run[r], mx), m_use = m_new == -INFINITY ? 0.0f : m_new;
-                corr[r] = fast_exp2(m_run[r] - m_use);
-                m_run[r] = m_new;
+                for (int j = 0; j < 8; j++) mx[r] = fmaxf(mx[r], fmaxf(sacc[j][2 * r], sacc[j][2 * r + 1]));
+            }
+            if (__any_sync(0xffffffffu, mx[0] > m_run[0] + 8.0f || mx[1] > m_run[1] + 8.0f)) {
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+                    mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+                    const float m_new = fmaxf(m_run[r], mx[r]), corr = fast_exp2(m_run[r] - (m_new == -INFINITY ? 0.0f : m_new));
+                    m_run[r] = m_new;
+                    l_run[r] *= corr;
+#pragma unroll
+                    for (int jd = 0; jd < 8; jd++) {
+                        oacc[jd][2 * r] *= corr;
+                        oacc[jd][2 * r + 1] *= corr;
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const float m_use = m_run[r] == -INFINITY ? 0.0f : m_run[r];
                 float sum = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
@@ -197,14 +213,7 @@ __global__ void __launch_bounds__(GROUPS * WARPS * 32, blocks_per_sm(GROUPS)) at
                     sacc[j][2 * r + 1] = fast_exp2(sacc[j][2 * r + 1] - m_use);
                     sum += sacc[j][2 * r] + sacc[j][2 * r + 1];
                 }
-                l_run[r] = l_run[r] * corr[r] + sum;  // this lane's share of the row; the quad's shares meet at the end
-            }
-#pragma unroll
-            for (int jd = 0; jd < 8; jd++) {
-                oacc[jd][0] *= corr[0];
-                oacc[jd][1] *= corr[0];
-                oacc[jd][2] *= corr[1];
-                oacc[jd][3] *= corr[1];
+                l_run[r] += sum;  // this lane's share of the row; the quad's shares meet at the end
             }
             // O += P V: key step kk = keys 16 kk .. 16 kk + 15 (one page); P's accumulators are the A fragments.
 #pragma unroll
