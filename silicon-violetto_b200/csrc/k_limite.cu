@@ -271,6 +271,57 @@ __global__ void __launch_bounds__(128) merge_kernel(const float* __restrict__ pa
     if (out_b) *reinterpret_cast<uint2*>(out_b + (size_t(t) * n_q + h) * D + d0) = make_uint2(pack_bf16(r.x, r.y), pack_bf16(r.z, r.w));  // for a tensor-core o projection
 }
 
+// The same for at most MERGE_FEW splits: a warp per (token, head), four to a block, all loads together, the sums in the same order
+// (so the same bits). A prompt's steps have two splits a row: a block a row of the kernel above left two of its four warps without
+// one, and put 5 120 blocks with a barrier each on the chip for 512 rows of 10 heads. Both bound by their few dependent trips
+// to L2 and by how many of them are in flight: 10 us there for the kernel above, 4 for this one (a prompt of 1 500 tokens through 48
+// layers 14.47 to 13.61 ms).
+constexpr uint32_t MERGE_FEW = 4;
+__global__ void __launch_bounds__(128) merge_few_kernel(const float* __restrict__ part, uint32_t max_splits, uint32_t n_items, uint32_t n_q, uint32_t n_kv,
+                                                        const float* __restrict__ vdir, const float* __restrict__ gates, const float* __restrict__ xsa, float* out,
+                                                        uint16_t* out_b) {
+    pdl_start();
+    const uint32_t item = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32, d0 = 4 * lane;
+    if (item >= n_items) return;
+    const uint32_t t = item / n_q, h = item - t * n_q;
+    const float* pp = part + size_t(item) * max_splits * PART;
+    float2 ml[MERGE_FEW];
+    float4 ov[MERGE_FEW], vd = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float xh = 0.0f, gt = 0.0f;
+#pragma unroll
+    for (uint32_t u = 0; u < MERGE_FEW; u++) {
+        ml[u] = make_float2(-INFINITY, 0.0f);
+        ov[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (u < max_splits) {
+            ml[u] = *reinterpret_cast<const float2*>(pp + u * PART);
+            ov[u] = *reinterpret_cast<const float4*>(pp + u * PART + 4 + d0);
+        }
+    }
+    if (vdir) {
+        vd = *reinterpret_cast<const float4*>(vdir + (size_t(t) * n_kv + h / (n_q / n_kv)) * D + d0);
+        xh = xsa[h];
+        gt = gates[item];
+    }
+    float mm = -INFINITY, ll = 0.0f;
+    float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (uint32_t u = 0; u < MERGE_FEW; u++) mm = fmaxf(mm, ml[u].x);
+#pragma unroll
+    for (uint32_t u = 0; u < MERGE_FEW; u++) {
+        if (ml[u].x == -INFINITY) continue;  // (the same for the whole warp)
+        const float wk = __expf(ml[u].x - mm);
+        ll += ml[u].y * wk;
+        r.x += ov[u].x * wk; r.y += ov[u].y * wk; r.z += ov[u].z * wk; r.w += ov[u].w * wk;
+    }
+    r.x /= ll; r.y /= ll; r.z /= ll; r.w /= ll;
+    if (vdir) {
+        const float pr = warp_sum(r.x * vd.x + r.y * vd.y + r.z * vd.z + r.w * vd.w), xs = xh * pr;
+        r = make_float4((r.x - xs * vd.x) * gt, (r.y - xs * vd.y) * gt, (r.z - xs * vd.z) * gt, (r.w - xs * vd.w) * gt);
+    }
+    *reinterpret_cast<float4*>(out + size_t(item) * D + d0) = r;
+    if (out_b) *reinterpret_cast<uint2*>(out_b + size_t(item) * D + d0) = make_uint2(pack_bf16(r.x, r.y), pack_bf16(r.z, r.w));  // for a tensor-core o projection
+}
+
 // kernels.metal:1663-1693 `kv_compact` over the local rings and the global pool. grid (runs, local + global layers), a warp
 // per kv head.
 __global__ void compact_kernel(const RunIn* __restrict__ runs, const uint32_t* __restrict__ path, const uint32_t* __restrict__ path_len, const uint32_t* __restrict__ lens,
@@ -353,7 +404,9 @@ void launch_limite_attn(const float* qkv, const uint32_t* meta, const uint32_t* 
     }
     if (by_tile) launch_limite_attn_rows(qkv, meta, tin, vis, tiles, k_cache, v_cache, kv, n_q, window, scale, n_tiles, kps, splits, part, s);
     else launch_limite_attn_mma(qkv, meta, tin, vis, k_cache, v_cache, kv, n_q, window, scale, n, kps, splits, part, s);
-    launch_pdl(limite::merge_kernel, dim3(n, n_q), 128, 0, s, part, splits, n_q, kv.n_kv, vdir, gates, xsa, out, out_b);
+    // At most four splits: a warp merges them all, whatever the rows; above, four warps share them out.
+    if (splits <= limite::MERGE_FEW) launch_pdl(limite::merge_few_kernel, (n * n_q + 3) / 4, 128, 0, s, part, splits, n * n_q, n_q, kv.n_kv, vdir, gates, xsa, out, out_b);
+    else launch_pdl(limite::merge_kernel, dim3(n, n_q), 128, 0, s, part, splits, n_q, kv.n_kv, vdir, gates, xsa, out, out_b);
 }
 void launch_limite_compact(const RunIn* runs, const uint32_t* path, const uint32_t* path_len, const uint32_t* lens, uint16_t* k_local, uint16_t* v_local,
                            uint16_t* k_global, uint16_t* v_global, const LimiteKv& local, const LimiteKv& global, uint32_t n_local, uint32_t n_global, uint32_t n_runs,

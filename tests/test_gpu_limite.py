@@ -119,6 +119,27 @@ def test_limite_forward_matches_the_oracle(model, keys_per_block):
     prod.close()
 
 
+@pytest.mark.parametrize("ctx,splits", [(40, 1), (100, 2), (240, 4), (258, 5)])
+def test_limite_splits_are_merged_by_a_warp_or_by_four(tmp_path, ctx, splits):
+    """Splits of 64 keys: up to four of them one warp merges a (token, head), four to a block; five take the kernel of four
+    warps. 1 row (10 items: two warps of the last block have none) and 3 rows of a tile (30). The tolerance is _step's."""
+    path = tmp_path / "limite.vlt"
+    desc = synth.write_limite(path, seed=6, **MODELS["5 layers, the reference's widths"])
+    prod, orc = _pair(path, E.Tuning(attn_keys_per_cta=64))
+    vr, rng = desc["vocab_real"], np.random.default_rng(ctx)
+    s = prod.new_seq()
+    assert orc.new_seq() == s
+    tokens = rng.integers(0, vr, ctx + 4).astype(np.uint32)
+    for i in range(0, ctx, 32):
+        r = [(s, tokens[i:min(i + 32, ctx)], E.Rows.NONE, False)]
+        prod.debug_step(r)
+        orc.step(r)
+    assert -(-(ctx + 9) // 64) == splits
+    for part in (tokens[ctx:ctx + 3], tokens[ctx + 3:]):
+        _step(prod, orc, [(s, part, E.Rows.ALL, False)], vr)
+    prod.close()
+
+
 def test_generator_on_the_reference_architecture_with_its_block_drafter(tmp_path):
     """The reference's own pairing: a target of its architecture (5 layers at its widths here) and its block drafter
     reading two of the target's layers, through the generator, beside a request behind the replay drafter and a plain
