@@ -222,55 +222,42 @@ void launch_attn_plain(const float* qkv, const uint32_t* meta, const uint32_t* t
 // ------------------------------------------------------------ split merge
 // kernels.metal:1314-1362 `attn_dec_reduce`, with a running maximum: the partials of a
 // (token, head) are (m, l, o[64]) per key split; out = sum(o_s 2^(m_s - M)) / sum(l_s 2^(m_s - M)).
-// One block per token and four heads, 64 threads a head.
 // Splits past a tile's keys hold m = -inf (the attention kernel writes every slot).
-// COMBINE_HEADS heads per block, 64 threads each: four when there are blocks enough to fill the GPU anyway (fewer,
-// fatter blocks schedule faster), one otherwise.
-template <uint32_t COMBINE_HEADS>
-__global__ void __launch_bounds__(64 * COMBINE_HEADS) attn_combine_kernel(const float* __restrict__ part, uint32_t max_splits, uint32_t n_heads, float* out,
-                                                                          uint16_t* out_b) {
+// At most COMBINE_FEW splits: half a warp per (token, head), four dims a lane, eight to a block, every load asked for at once: bound
+// by one trip to L2 and by the bytes. Before, 64 threads a head met
+// twice at block barriers for the statistics: a verify step of 160 rows, 32 heads, 16 layers 2 848 us, now 2 812; of 40 rows as before.
+constexpr uint32_t COMBINE_FEW = 8;
+__global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restrict__ part, uint32_t max_splits, uint32_t n_items, float* out, uint16_t* out_b) {
     pdl_start();
-    __shared__ float ws[COMBINE_HEADS][64];   // the splits' weights 2^(m_s - M), 0 for an empty split
-    __shared__ float lws[COMBINE_HEADS][64];  // l_s times that
-    __shared__ float red[COMBINE_HEADS][2];
-    const uint32_t t = blockIdx.x, hl = threadIdx.x / 64, h = blockIdx.y * COMBINE_HEADS + hl, d = threadIdx.x % 64;
-    const bool live = h < n_heads;
-    const float* pp = part + (size_t(t) * n_heads + (live ? h : 0)) * max_splits * ATTN_PART;
-    // A thread per split for the statistics (at most 64 splits, engine.cu `attention_split`), then a thread
-    // per dim with the splits' loads independent of each other.
-    // The first eight splits' values are asked for together with the statistics (they do not depend on them): one
-    // round trip to L2 instead of two.
-    float v8[8];
+    const uint32_t item = blockIdx.x * 8 + threadIdx.x / 16, d = 4 * (threadIdx.x % 16);
+    if (item >= n_items) return;
+    const float* pp = part + size_t(item) * max_splits * ATTN_PART;
+    float2 ml[COMBINE_FEW];
+    float4 v[COMBINE_FEW];
 #pragma unroll
-    for (uint32_t s = 0; s < 8; s++) v8[s] = s < max_splits ? pp[s * ATTN_PART + 4 + d] : 0.0f;
-    const bool has = d < max_splits;
-    const float ms = has ? pp[d * ATTN_PART] : -INFINITY;
-    const float ls = has ? pp[d * ATTN_PART + 1] : 0.0f;
-    float mm = ms;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    if (d % 32 == 0) red[hl][d / 32] = mm;
-    __syncthreads();
-    mm = fmaxf(red[hl][0], red[hl][1]);
-    const float w = ms == -INFINITY ? 0.0f : exp2f(ms - mm);
-    ws[hl][d] = w;
-    lws[hl][d] = ls * w;  // summed in split order below, so that the result does not depend on the warp layout
-    __syncthreads();
-    float ll = 0.0f, oo = 0.0f;
-    for (uint32_t s = 0; s < max_splits; s++) ll += lws[hl][s];
-#pragma unroll
-    for (uint32_t s = 0; s < 8; s++)  // an empty split's o was never written: whatever is there must not count
-        if (s < max_splits) oo += ws[hl][s] == 0.0f ? 0.0f : v8[s] * ws[hl][s];
-#pragma unroll 8
-    for (uint32_t s = 8; s < max_splits; s++) {
-        const float v = pp[s * ATTN_PART + 4 + d];
-        oo += ws[hl][s] == 0.0f ? 0.0f : v * ws[hl][s];
+    for (uint32_t s = 0; s < COMBINE_FEW; s++) {
+        ml[s] = make_float2(-INFINITY, 0.0f);
+        v[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (s < max_splits) {
+            ml[s] = *reinterpret_cast<const float2*>(pp + s * ATTN_PART);
+            v[s] = *reinterpret_cast<const float4*>(pp + s * ATTN_PART + 4 + d);
+        }
     }
-    if (!live) return;
-    const float r = oo / ll;
-    const size_t at = size_t(t) * n_heads * 64 + h * 64 + d;
-    out[at] = r;
-    if (out_b) out_b[at] = f32_to_bf16(r);
+    float mm = -INFINITY, ll = 0.0f, o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (uint32_t s = 0; s < COMBINE_FEW; s++) mm = fmaxf(mm, ml[s].x);
+#pragma unroll
+    for (uint32_t s = 0; s < COMBINE_FEW; s++) {
+        if (s >= max_splits) break;
+        const float w = ml[s].x == -INFINITY ? 0.0f : exp2f(ml[s].x - mm);
+        ll = __fadd_rn(ll, __fmul_rn(ml[s].y, w));
+        if (w == 0.0f) continue;  // an empty split's o was never written: whatever is there must not count
+        o[0] += v[s].x * w; o[1] += v[s].y * w; o[2] += v[s].z * w; o[3] += v[s].w * w;
+    }
+    const float4 r = make_float4(o[0] / ll, o[1] / ll, o[2] / ll, o[3] / ll);
+    const size_t at = size_t(item) * 64 + d;
+    *reinterpret_cast<float4*>(out + at) = r;
+    if (out_b) *reinterpret_cast<uint2*>(out_b + at) = make_uint2(pack_bf16(r.x, r.y), pack_bf16(r.z, r.w));
 }
 
 // The same merge for many splits (a long context read by few streams): one block per (token, head), four groups of 64
@@ -320,9 +307,8 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float* __r
 }
 
 void launch_attn_combine(const AttnArgs& a, cudaStream_t s) {
-    if (a.max_splits > 8) launch_pdl(attn_combine_wide_kernel, dim3(a.n, a.n_heads), 256, 0, s, a.part, a.max_splits, a.n_heads, a.out, a.out_b);
-    else if (a.n * a.n_heads >= 2048) launch_pdl(attn_combine_kernel<4>, dim3(a.n, (a.n_heads + 3) / 4), 256, 0, s, a.part, a.max_splits, a.n_heads, a.out, a.out_b);
-    else launch_pdl(attn_combine_kernel<1>, dim3(a.n, a.n_heads), 64, 0, s, a.part, a.max_splits, a.n_heads, a.out, a.out_b);
+    if (a.max_splits > COMBINE_FEW) launch_pdl(attn_combine_wide_kernel, dim3(a.n, a.n_heads), 256, 0, s, a.part, a.max_splits, a.n_heads, a.out, a.out_b);
+    else launch_pdl(attn_combine_kernel, (a.n * a.n_heads + 7) / 8, 128, 0, s, a.part, a.max_splits, a.n * a.n_heads, a.out, a.out_b);
 }
 
 // ------------------------------------------------------------- row preparation
