@@ -187,6 +187,27 @@ def test_two_attention_kernels_agree_at_long_context(keys_per_block):
     assert err < 2e-2, err
 
 
+@pytest.mark.parametrize("keys_per_block,splits", [(4000, 1), (352, 8), (312, 9)])
+def test_split_merges_agree_with_the_scalar_attention_where_the_forms_change(keys_per_block, splits):
+    """One split, the most that half a warp merges and the fewest that a block does; 13 rows of 4 heads leave the last block of
+    the first form half empty. The tolerance is the one of the two attention kernels above."""
+    w = util.weights("micro", 0)
+    cfg = E.EngineConfig(max_seqs=3, max_step_tokens=32, max_chunk=8, global_kv_tokens=3 * 3008, max_seq_len=3008, max_head_rows=24)
+    outs = []
+    for plain in (False, True):
+        eng = E.Engine(w, cfg, E.Tuning(plain_attention=plain, attn_keys_per_cta=keys_per_block))
+        seqs = [eng.new_seq() for _ in range(3)]
+        for i, s in enumerate(seqs):
+            eng.bench_fill(s, [2800, 17, 1234][i], seed=5 + i)
+        runs = [(s, [3 + i, 9, 100 + i, 7, 200][: [5, 3, 5][i]], E.Rows.ALL, False) for i, s in enumerate(seqs)]
+        outs.append(eng.debug_step(runs, E.StepOptions(read_logits=True)).logits)
+        if not plain:
+            assert list(eng.debug_read("attn_split"))[1] == splits
+        eng.close()
+    err = float(np.abs(outs[0] - outs[1]).max())
+    assert err < 2e-2, err
+
+
 def test_verify_runs_with_the_replay_drafter_match_the_oracle():
     """Chain verification: the replay drafter's drafts (some wrong), accept, lens, feed, emitted."""
     prod, orc = pair("micro", None)
